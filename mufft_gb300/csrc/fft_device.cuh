@@ -17,7 +17,11 @@
 
 #include <cooperative_groups.h>
 
+#include <cstddef>
+#include <type_traits>
+
 #include "common.h"
+#include "registry.h"
 
 namespace mgb {
 
@@ -223,9 +227,14 @@ __device__ __forceinline__ void tile_sync()
 
 // Twiddle multiply and DFT of stage s on the thread's R registers.
 // Register u*r + m holds input m of butterfly i = j*B + tl + TL*u.
-template <int L, int R, int Q, int s>
-__device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, const float2 *__restrict__ tw)
+// BASE (stages after the first): every output also times `base`, carried by
+// the twiddles -- the DFT is linear -- for r + 1 products per butterfly less
+// the r of a multiply of its outputs.
+template <int L, int R, int Q, int s, bool BASE = false>
+__device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, const float2 *__restrict__ tw,
+                                              float2 base = float2{})
 {
+    static_assert(!BASE || s > 0, "the first stage has no twiddles to carry the factor");
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
     constexpr int r = S::radix(s), p = S::pbefore(s), NB = R / r;
@@ -244,17 +253,31 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, con
                 w[4] = make_float2(b.x, b.y);
                 w[8] = make_float2(b.z, b.w);
             }
-            // remaining powers: at most three rounded products deep
+            if constexpr (BASE) {
+                // base * W^(mk): base, then each power from one half as long
+                float2 z[r];
+                z[0] = base;
 #pragma unroll
-            for (int m = 3; m < r; m++) {
-                if (m == 4 || m == 8)
-                    continue;
-                const int hi = m >= 8 ? 8 : (m >= 4 ? 4 : 2);
-                w[m] = cmul(w[m - hi], w[hi]);
+                for (int m = 1; m < r; m++) {
+                    const int hi = m >= 8 ? 8 : (m >= 4 ? 4 : (m >= 2 ? 2 : 1));
+                    z[m] = cmul(z[m - hi], w[hi]);
+                }
+#pragma unroll
+                for (int m = 0; m < r; m++)
+                    v[u * r + m] = cmul(v[u * r + m], z[m]);
+            } else {
+                // remaining powers: at most three rounded products deep
+#pragma unroll
+                for (int m = 3; m < r; m++) {
+                    if (m == 4 || m == 8)
+                        continue;
+                    const int hi = m >= 8 ? 8 : (m >= 4 ? 4 : 2);
+                    w[m] = cmul(w[m - hi], w[hi]);
+                }
+#pragma unroll
+                for (int m = 1; m < r; m++)
+                    v[u * r + m] = cmul(v[u * r + m], w[m]);
             }
-#pragma unroll
-            for (int m = 1; m < r; m++)
-                v[u * r + m] = cmul(v[u * r + m], w[m]);
         }
         Dft<r>::run(&v[u * r]);
     }
@@ -344,6 +367,10 @@ __device__ __forceinline__ float2 c2r_fixup(float2 a, float2 bm, float2 w)
     return cadd(cadd(a, b), cmul(csub(a, b), w));
 }
 
+template <int V> struct Int {
+    static constexpr int value = V;
+};
+
 // Stage-0 load: register u*r + m <- element p = j*B + tl + TL*u + m*Q*B of
 // transform `tr`.  ALONG loads have unit stride (the planner only builds them
 // that way), so addresses are a base plus constant offsets.
@@ -389,7 +416,39 @@ __device__ __forceinline__ void st_policy(float2 *p, float2 v, unsigned long lon
                  : "memory");
 }
 
-template <int L, int R, int Q, int LMAP, bool COH = false>
+// Flavours of a tile kernel: which prologue and epilogue it carries.  FL_ANY
+// decides both at run time, with every form compiled in; the others fix them,
+// so that a launch pays no per-element tests and holds less code.  All of
+// them read whole plain inputs (PRO_PLAIN, no `half`).
+enum Flavour : int {
+    FL_ANY = 0,
+    FL_PLAIN = 1,   // EPI_PLAIN
+    FL_COLPOW = 2,  // EPI_TWIDDLE with tw_colpow
+    FL_BYROW = 3,   // EPI_TWIDDLE with tw_by_y
+    FL_R2C = 4,     // EPI_R2C
+};
+template <int FL> __device__ __forceinline__ int fl_prologue(const TileArgs &a)
+{
+    return FL == FL_ANY ? a.prologue : (int)PRO_PLAIN;
+}
+template <int FL> __device__ __forceinline__ int fl_half(const TileArgs &a) { return FL == FL_ANY ? a.half : 0; }
+template <int FL> __device__ __forceinline__ int fl_epilogue(const TileArgs &a)
+{
+    return FL == FL_ANY      ? a.epilogue
+           : FL == FL_PLAIN  ? (int)EPI_PLAIN
+           : FL == FL_R2C    ? (int)EPI_R2C
+                             : (int)EPI_TWIDDLE;
+}
+template <int FL> __device__ __forceinline__ bool fl_byrow(const TileArgs &a)
+{
+    return FL == FL_ANY ? a.tw_by_y != 0 : FL == FL_BYROW;
+}
+template <int FL> __device__ __forceinline__ bool fl_colpow(const TileArgs &a)
+{
+    return FL == FL_ANY ? a.tw_colpow != 0 : FL == FL_COLPOW;
+}
+
+template <int L, int R, int Q, int LMAP, bool COH = false, int FL = FL_ANY>
 __device__ __forceinline__ void load_stage0(const TileArgs &a, const float2 *__restrict__ in,
                                             const float2 *__restrict__ in2, unsigned tr, int j, int tl,
                                             float2 (&v)[R])
@@ -397,34 +456,48 @@ __device__ __forceinline__ void load_stage0(const TileArgs &a, const float2 *__r
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
     constexpr int r = S::radix(0), NB = R / r, B = TT::B(0), TL = TT::TL;
+    const int mlim = fl_half<FL>(a) ? r / 2 : r;  // zero-padded upper half: inputs m >= r/2 stay zero
+    // (zeroed up front by the kernels of many forms: a zeroing under the tests
+    // made the ragged kernels spill kilobytes)
+    if (FL == FL_ANY || tr >= a.ntrans) {
 #pragma unroll
-    for (int q = 0; q < R; q++)
-        v[q] = make_float2(0.f, 0.f);
+        for (int q = 0; q < R; q++)
+            v[q] = make_float2(0.f, 0.f);
+    }
     if (tr >= a.ntrans)
         return;
-    const int mlim = a.half ? r / 2 : r;  // zero-padded upper half: inputs m >= r/2 stay zero
     const long long tbase = (long long)tr * a.in_dist;
     const long long p0 = (long long)j * B + tl;  // position of register 0
     const long long sst = (LMAP == ALONG) ? 1 : a.in_stride;
     const float2 *f = in + tbase + p0 * sst;
-    switch (a.prologue) {
+    switch (fl_prologue<FL>(a)) {
     case PRO_PLAIN: {
         // read-only loads carry an L2 policy: evict-first for a pass that
-        // streams its input, else evict-normal
+        // streams its input, else evict-normal.  One uniform test decides
+        // whether the upper half is read: the loads themselves carry none.
         unsigned long long pol = 0;
         if constexpr (!COH)
             pol = (a.l2 & L2_LOAD_FIRST) ? l2_evict_first() : l2_evict_normal();
+        const long long mstep = (long long)(Q * B) * sst, ustep = (long long)TL * sst;
+        auto fetch = [&](auto mcount) {
+            constexpr int MC = decltype(mcount)::value;
 #pragma unroll
-        for (int u = 0; u < NB; u++)
+            for (int u = 0; u < NB; u++) {
+                const float2 *src = f + u * ustep;
 #pragma unroll
-            for (int m = 0; m < r; m++)
-                if (m < mlim) {
-                    const float2 *src = f + (long long)(TL * u + m * Q * B) * sst;
+                for (int m = 0; m < MC; m++) {
                     if constexpr (COH)
                         v[u * r + m] = gload<COH>(src);
                     else
                         v[u * r + m] = ld_policy(src, pol);
+                    src += mstep;
                 }
+            }
+        };
+        if (mlim == r)
+            fetch(Int<r>{});
+        else
+            fetch(Int<r / 2>{});
         break;
     }
     case PRO_MUL: {
@@ -493,43 +566,58 @@ __device__ __forceinline__ void load_stage0_c2r_rows(const TileArgs &a, const fl
     using S = Sched<L, R>;
     using TT = Tile<L, R, 1>;
     constexpr int r = S::radix(0), NB = R / r, B = TT::B(0), TL = TT::TL;
+    constexpr bool CONST_PAD = B % 16 == 0 && (NB == 1 || TL % 16 == 0);
+    auto off = [](int u, int m) { return TL * u + B * m; };
     const bool valid = tr < a.ntrans;
     const bool mul = a.prologue == PRO_MUL_C2R;
-    const long long tbase = (long long)tr * a.in_dist;
-    auto fetch = [&](long long n) {
-        float2 xv = gload<COH>(in + tbase + n);
-        if (mul) {
-            float2 g = gload<COH>(in2 + ((a.in2_bcast & 2) ? 0 : tbase) + n);
-            g.y = a.conj2 ? -g.y : g.y;
-            xv = cscale(cmul(xv, g), a.scale);
-        }
-        return xv;
-    };
-    // X[M], the mirror of position 0, is loaded with the staged values so
-    // that its latency is not paid after the barrier
+    const float2 *f = in + (long long)tr * a.in_dist;
+    // X[M], the mirror of position 0, is loaded with the row so that its
+    // latency is not paid after the barrier
     float2 xm = make_float2(0.f, 0.f);
     if (valid) {
 #pragma unroll
-        for (int i = 0; i < R; i++)
-            region[padpos(tl + TL * i)] = fetch(tl + TL * i);
+        for (int q = 0; q < R; q++)
+            v[q] = gload<COH>(f + tl + off(q / r, q % r));
         if (tl == 0)
-            xm = fetch(L);
+            xm = gload<COH>(f + L);
+        if (mul) {
+            const float2 *g = in2 + ((a.in2_bcast & 2) ? 0 : (long long)tr * a.in_dist);
+            const float cs = a.conj2 ? -1.f : 1.f;
+            auto times = [&](float2 x, float2 y) {
+                y.y *= cs;
+                return cscale(cmul(x, y), a.scale);
+            };
+#pragma unroll
+            for (int q = 0; q < R; q++)
+                v[q] = times(v[q], gload<COH>(g + tl + off(q / r, q % r)));
+            if (tl == 0)
+                xm = times(xm, gload<COH>(g + L));
+        }
+        const int base = padpos(tl);
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            region[CONST_PAD ? base + off(q / r, q % r) / 16 * 17 : padpos(tl + off(q / r, q % r))] = v[q];
+    } else {
+#pragma unroll
+        for (int q = 0; q < R; q++)
+            v[q] = make_float2(0.f, 0.f);
     }
     __syncthreads();
-#pragma unroll
-    for (int q = 0; q < R; q++)
-        v[q] = make_float2(0.f, 0.f);
     if (valid) {
+        // the mirror of position tl + o is L - tl - o: a base less a constant
+        // where the offsets o are multiples of the padding's 16
+        const float2 *w = a.rtw + tl;
+        const int mp = padpos(L - tl);
 #pragma unroll
-        for (int u = 0; u < NB; u++)
-#pragma unroll
-            for (int m = 0; m < r; m++) {
-                const int local = tl + TL * u + m * B;
-                const float2 xa = region[padpos(local)];
-                // only register 0 of thread 0 is position 0 (its mirror X[M] is not staged)
-                const float2 xb = (u == 0 && m == 0 && tl == 0) ? xm : region[padpos(L - local)];
-                v[u * r + m] = c2r_fixup(xa, xb, __ldg(&a.rtw[local]));
-            }
+        for (int q = 0; q < R; q++) {
+            const int o = off(q / r, q % r);
+            float2 xb;
+            if (q == 0 && tl == 0)
+                xb = xm;  // its mirror X[M] is not staged
+            else
+                xb = region[CONST_PAD ? mp - o / 16 * 17 : padpos(L - tl - o)];
+            v[q] = c2r_fixup(v[q], xb, __ldg(w + o));
+        }
     }
     if (a.conj & 1) {
 #pragma unroll
@@ -634,9 +722,10 @@ __host__ __device__ constexpr size_t tile_smem_bytes()
 
 // --------------------------------------------------------------- kernel
 
-template <int L, int R, int C, int Q, int LMAP, int SMAP, int s>
+// BASE: the outputs times `base` (stage_compute), in the last stage.
+template <int L, int R, int C, int Q, int LMAP, int SMAP, int s, bool BASE = false>
 __device__ __forceinline__ void run_stages(float2 (&v)[R], int j, int &c, int &tl, float2 *smem,
-                                           const float2 *__restrict__ tw)
+                                           const float2 *__restrict__ tw, float2 base = float2{})
 {
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
@@ -648,8 +737,8 @@ __device__ __forceinline__ void run_stages(float2 (&v)[R], int j, int &c, int &t
         stage_read<L, R, Q, s>(smem + c * RS, v, j, tl);
         if (s < S::NST - 1)
             tile_sync<Q>();
-        stage_compute<L, R, Q, s>(v, j, tl, tw);
-        run_stages<L, R, C, Q, LMAP, SMAP, s + 1>(v, j, c, tl, smem, tw);
+        stage_compute<L, R, Q, s, BASE && s == S::NST - 1>(v, j, tl, tw, base);
+        run_stages<L, R, C, Q, LMAP, SMAP, s + 1, BASE>(v, j, c, tl, smem, tw, base);
     }
 }
 
@@ -673,7 +762,7 @@ template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_min
 // TAB: every transform of the tile has its own buffers (in_tab / in2_tab /
 // out_tab, distances 0): a tile of C unrelated requests of one size.
 template <int L, int R, int C, int Q, int LMAP, int SMAP, bool COH, bool SIN = false, bool PRE = false,
-          bool C2RS = false, bool EMUL = false, bool TAB = false>
+          bool C2RS = false, bool EMUL = false, bool TAB = false, int FL = FL_ANY>
 __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int j, long long ioff, long long ooff,
                                           float2 *smem, const float2 *sin = nullptr, unsigned twy = 0,
                                           const float2 *pre = nullptr)
@@ -709,17 +798,19 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
     } else if constexpr (TAB) {
         const unsigned t = tile0 + c;
         const bool ok = t < a.ntrans;
-        load_stage0<L, R, Q, LMAP, COH>(a, ok ? a.in_tab[t] : in, (ok && a.in2_tab) ? a.in2_tab[t] : in2, t, j, tl,
-                                        v);
+        load_stage0<L, R, Q, LMAP, COH, FL>(a, ok ? a.in_tab[t] : in, (ok && a.in2_tab) ? a.in2_tab[t] : in2, t, j,
+                                            tl, v);
     } else {
-        load_stage0<L, R, Q, LMAP, COH>(a, in, in2, tile0 + c, j, tl, v);
+        load_stage0<L, R, Q, LMAP, COH, FL>(a, in, in2, tile0 + c, j, tl, v);
     }
+    const int epilogue = fl_epilogue<FL>(a);
+    const bool byrow = fl_byrow<FL>(a), colpow = fl_colpow<FL>(a);
     // The four-step twiddle region, and this thread's column-power base, are
     // computed while the stage-0 loads are in flight (the epilogue reads the
     // region after the exchanges' barriers).
     float2 wbase = make_float2(1.f, 0.f);
     if constexpr (tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
-        if (a.epilogue == EPI_TWIDDLE && a.tw_colpow && !a.tw_by_y) {
+        if (epilogue == EPI_TWIDDLE && colpow && !byrow) {
             int cl, tll;  // the thread's transform and position in the last stage
             split_tid<SMAP, C, TL>(threadIdx.x, cl, tll);
             wbase = fourstep_twiddle((unsigned)(j * TT::B(NST - 1) + tll) * (tile0 + cl), a.tw_scale, a.tw_mask);
@@ -727,13 +818,13 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
     }
     if constexpr (tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
         float2 *thi = smem + tile_exchange_bytes<L, R, C, Q, LMAP, SMAP>() / sizeof(float2);
-        if (a.epilogue == EPI_TWIDDLE && a.tw_by_y) {
+        if (epilogue == EPI_TWIDDLE && byrow) {
             // W_N^(k*row) for every output k, the same for all columns
             for (int k = threadIdx.x; k < L; k += tile_threads<L, R, C, Q>())
                 thi[k] = fourstep_twiddle((unsigned)k * twy, a.tw_scale, a.tw_mask);
             if constexpr (NST == 1)
                 __syncthreads();
-        } else if (a.epilogue == EPI_TWIDDLE && a.tw_colpow) {
+        } else if (epilogue == EPI_TWIDDLE && colpow) {
             // W_N^(col*off_i), col = tile*C + c, for the last stage's output
             // offsets off_i = TL*u + m*BL of register i = u*rl + m
             constexpr int rl = S::radix(NST - 1), BL = TT::B(NST - 1);
@@ -744,7 +835,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
             }
             if constexpr (NST == 1)
                 __syncthreads();
-        } else if (a.epilogue == EPI_TWIDDLE && a.tw_lo) {
+        } else if (epilogue == EPI_TWIDDLE && FL == FL_ANY && a.tw_lo) {
             // Four-step twiddle, per-tile half: W_N^(k*C*tile) for every output k
             // (the per-column half W_N^(k*c) comes from the plan's table tw_lo).
             for (int k = threadIdx.x; k < L; k += tile_threads<L, R, C, Q>())
@@ -754,7 +845,10 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
         }
     }
     stage_compute<L, R, Q, 0>(v, j, tl, a.tw);
-    run_stages<L, R, C, Q, LMAP, SMAP, 1>(v, j, c, tl, smem, a.tw);
+    // the column powers' base rides in the last stage's twiddles where the
+    // kernel has that one epilogue
+    constexpr bool BASE = FL == FL_COLPOW && NST > 1;
+    run_stages<L, R, C, Q, LMAP, SMAP, 1, BASE>(v, j, c, tl, smem, a.tw, wbase);
     // No CTA of the cluster may leave while others still read its slice.
     if constexpr (Q > 1)
         cg::this_cluster().barrier_arrive();
@@ -770,12 +864,13 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
             out = a.out_tab[tr];
     }
 
-    if (a.epilogue == EPI_R2C || a.epilogue == EPI_R2C_FULL) {
+    if (epilogue == EPI_R2C || epilogue == EPI_R2C_FULL) {
         // Z[k] and Z[L-k] sit in different threads (and CTAs): scatter the
         // outputs to their owners' slices, then every CTA resolves its own
         // range of k, reading Z[L-k] wherever it lives.
         constexpr int M = L, LQ = TT::LQ;
-        const bool full = a.epilogue == EPI_R2C_FULL;
+        const bool full = epilogue == EPI_R2C_FULL;
+        const long long os = SMAP == ALONG ? 1 : a.out_stride;
         if constexpr (NST > 1) {
             float2 *region = smem + c * RS;
             if constexpr (Q > 1)
@@ -797,11 +892,16 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                 // symmetry of a real input's spectrum, X[M-k] = conj(hi) (and
                 // X[M+k] = hi, X[2M-k] = conj(lo) for the full output), so a
                 // thread resolves k < M/2 and reads each value once.
-                const long long os = a.out_stride;
+                // Positions k and M - k are a base plus and less a constant
+                // where TL is a multiple of the padding's 16.
+                constexpr bool CP = TL % 16 == 0;
+                const int kp = padpos(tl), mp = padpos(M - tl);
+                float2 *olo = out + obase + (long long)tl * os, *ohi = out + obase + (long long)(M - tl) * os;
+                const float2 *rt = a.rtw + tl;
 #pragma unroll
                 for (int q = 0; q < R / 2; q++) {
                     const int k = tl + TL * q;
-                    const float2 zk = region[padpos(k)];
+                    const float2 zk = region[CP ? kp + TL * q / 16 * 17 : padpos(k)];
                     if (k == 0) {
                         out[obase] = make_float2(zk.x + zk.y, 0.f);
                         out[obase + (long long)M * os] = make_float2(zk.x - zk.y, 0.f);
@@ -813,12 +913,13 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                             out[obase + (long long)(M / 2 + M) * os] = hi;
                     } else {
                         float2 lo, hi;
-                        r2c_bins(zk, region[padpos(M - k)], __ldg(&a.rtw[k]), lo, hi);
-                        out[obase + (long long)k * os] = lo;
-                        out[obase + (long long)(M - k) * os] = cconj(hi);
+                        const float2 zm = region[CP ? mp - TL * q / 16 * 17 : padpos(M - k)];
+                        r2c_bins(zk, zm, __ldg(rt + TL * q), lo, hi);
+                        olo[(long long)(TL * q) * os] = lo;
+                        ohi[-(long long)(TL * q) * os] = cconj(hi);
                         if (full) {
-                            out[obase + (long long)(k + M) * os] = hi;
-                            out[obase + (long long)(2 * M - k) * os] = cconj(lo);
+                            olo[(long long)(TL * q + M) * os] = hi;
+                            ohi[(long long)(M - TL * q) * os] = cconj(lo);
                         }
                     }
                 }
@@ -904,55 +1005,74 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
     if (valid) {
         const long long sst = (SMAP == ALONG) ? 1 : a.out_stride;
         float2 *o0 = out + obase + (long long)p0 * sst;
-        if (a.epilogue == EPI_TWIDDLE) {
+        const long long mstep = (long long)(Q * BL) * sst, ustep = (long long)TL * sst;
+        // Output by output: a factor w(i, off) for register i at offset off
+        // (none: nullptr) and the store, so that the stores spread over the
+        // products.  Every test is uniform and outside these loops; the sign of
+        // a conjugated output is one too in the kernels of one form, and a
+        // factor in those of many (less code).
+        auto emit_signed = [&](auto w, auto sign) {
+#pragma unroll
+            for (int u = 0; u < NBL; u++) {
+                float2 *dst = o0 + u * ustep;
+#pragma unroll
+                for (int m = 0; m < rl; m++) {
+                    float2 y = v[u * rl + m];
+                    if constexpr (!std::is_same<decltype(w), std::nullptr_t>::value)
+                        y = cmul(y, w(u * rl + m, TL * u + m * Q * BL));
+                    if constexpr (EMUL)
+                        y = cscale(y, a.scale);
+                    st_policy(dst, sign(y), stpol);
+                    dst += mstep;
+                }
+            }
+        };
+        auto emit = [&](auto w) {
+            if constexpr (FL == FL_ANY) {
+                const float sg = (a.conj & 2) ? -1.f : 1.f;
+                emit_signed(w, [sg](float2 y) { return make_float2(y.x, sg * y.y); });
+            } else if (a.conj & 2) {
+                emit_signed(w, [](float2 y) { return cconj(y); });
+            } else {
+                emit_signed(w, [](float2 y) { return y; });
+            }
+        };
+        if (epilogue == EPI_TWIDDLE) {
             // W_N^(k*n) for output k of column n = tile*C + c: the column-power
             // base W_N^(p0*n) (wbase) times the region's W_N^(n*off) (filled
             // while the stage-0 loads were in flight, after the exchange slices)
-            float2 *thi = smem + tile_exchange_bytes<L, R, C, Q, LMAP, SMAP>() / sizeof(float2);
-#pragma unroll
-            for (int u = 0; u < NBL; u++)
-#pragma unroll
-                for (int m = 0; m < rl; m++) {
-                    const int off = TL * u + m * Q * BL;
-                    const int k = p0 + off;
-                    float2 w;
-                    if constexpr (tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
-                        if (a.tw_by_y)
-                            w = thi[k];
-                        else if (a.tw_colpow)
-                            w = cmul(wbase, thi[(u * rl + m) * C + c]);
-                        else if (a.tw_lo)
-                            w = cmul(__ldg(&a.tw_lo[k * C + c]), thi[k]);
-                        else
-                            w = fourstep_twiddle((unsigned)k * tr, a.tw_scale, a.tw_mask);
-                    } else {
-                        w = fourstep_twiddle((unsigned)k * (a.tw_by_y ? twy : tr), a.tw_scale, a.tw_mask);
-                    }
-                    float2 y = cmul(v[u * rl + m], w);
-                    if (a.conj & 2)
-                        y.y = -y.y;
-                    st_policy(&o0[(long long)off * sst], y, stpol);
-                }
+            const float2 *thi = smem + tile_exchange_bytes<L, R, C, Q, LMAP, SMAP>() / sizeof(float2);
+            if constexpr (tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
+                if (byrow)
+                    emit([&](int, int off) { return thi[p0 + off]; });
+                else if (BASE)
+                    emit([&](int i, int) { return thi[i * C + c]; });
+                else if (colpow)
+                    emit([&](int i, int) { return cmul(wbase, thi[i * C + c]); });
+                else if (a.tw_lo)
+                    emit([&](int, int off) { return cmul(__ldg(&a.tw_lo[(p0 + off) * C + c]), thi[p0 + off]); });
+                else
+                    emit([&](int, int off) {
+                        return fourstep_twiddle((unsigned)(p0 + off) * tr, a.tw_scale, a.tw_mask);
+                    });
+            } else {
+                const unsigned col = byrow ? twy : tr;
+                emit([&](int, int off) {
+                    return fourstep_twiddle((unsigned)(p0 + off) * col, a.tw_scale, a.tw_mask);
+                });
+            }
+        } else if constexpr (EMUL) {
+            const float2 *e = a.in2 + (long long)tr * a.in2_dist + (long long)p0 * a.in2_stride;
+            emit([&](int, int off) { return __ldg(e + (long long)off * a.in2_stride); });
         } else {
-            const float sg = (a.conj & 2) ? -1.f : 1.f;
-#pragma unroll
-            for (int u = 0; u < NBL; u++)
-#pragma unroll
-                for (int m = 0; m < rl; m++) {
-                    const int off = TL * u + m * Q * BL;
-                    float2 y = v[u * rl + m];
-                    if constexpr (EMUL)
-                        y = cscale(cmul(y, __ldg(&a.in2[(long long)tr * a.in2_dist + (long long)(p0 + off) * a.in2_stride])),
-                                   a.scale);
-                    st_policy(&o0[(long long)off * sst], make_float2(y.x, sg * y.y), stpol);
-                }
+            emit(nullptr);
         }
     }
     if constexpr (Q > 1)
         cg::this_cluster().barrier_wait();
 }
 
-template <int L, int R, int C, int Q, int LMAP, int SMAP>
+template <int L, int R, int C, int Q, int LMAP, int SMAP, int FL = FL_ANY>
 __global__ void __launch_bounds__(tile_threads<L, R, C, Q>(), tile_min_blocks<L, R, C, Q>()) tile_fft(const TileArgs a)
 {
     extern __shared__ float2 smem[];
@@ -971,11 +1091,13 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, Q>(), tile_min_blocks<L,
         j = (int)cg::this_cluster().block_rank();
         tile = blockIdx.x / Q;
     }
-    tile_body<L, R, C, Q, LMAP, SMAP, false>(a, tile, j, ioff, ooff, smem, nullptr, blockIdx.y);
+    tile_body<L, R, C, Q, LMAP, SMAP, false, false, false, false, false, false, FL>(a, tile, j, ioff, ooff, smem, nullptr,
+                                                                                   blockIdx.y);
 }
 
 // Row tile whose c2r fix-up prologue stages each row in shared memory
-// (load_stage0_c2r_rows); one CTA per tile as tile_fft.
+// (load_stage0_c2r_rows) and whose stores are plain; one CTA per tile as
+// tile_fft.
 template <int L, int R, int C>
 __global__ void __launch_bounds__(tile_threads<L, R, C, 1>(), tile_min_blocks<L, R, C, 1>())
     tile_fft_c2r_rows(const TileArgs a)
@@ -990,7 +1112,8 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, 1>(), tile_min_blocks<L,
         ioff = (long long)blockIdx.y * a.in_batch;
         ooff = (long long)blockIdx.y * a.out_batch;
     }
-    tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, true>(a, blockIdx.x, 0, ioff, ooff, smem);
+    tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, true, false, false, FL_PLAIN>(a, blockIdx.x, 0, ioff, ooff,
+                                                                                           smem);
 }
 
 // The staged-c2r variant of a row tile, or null where there is none.
@@ -1000,6 +1123,22 @@ template <int L, int R, int C, int Q> constexpr const void *tile_c2r_rows_fn()
         return (const void *)&tile_fft_c2r_rows<L, R, C>;
     else
         return nullptr;
+}
+
+// The flavoured forms of a tile (registry.h), null where there is none.
+template <int L, int R, int C, int Q, int LMAP, int SMAP> constexpr TileFlavours tile_flavours()
+{
+    TileFlavours f{};
+    if constexpr (Q == 1) {
+        f.plain = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_PLAIN>;
+        if constexpr (LMAP == ACROSS && SMAP == ACROSS && tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
+            f.colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_COLPOW>;
+            f.byrow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_BYROW>;
+        }
+        if constexpr (LMAP == ALONG && SMAP == ALONG)
+            f.r2c = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_R2C>;
+    }
+    return f;
 }
 
 }  // namespace mgb

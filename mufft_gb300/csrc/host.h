@@ -208,6 +208,9 @@ bool attach_tma(std::vector<Pass> &ps, PlanResources &res, bool dry, int device)
 bool attach_stream(std::vector<Pass> &ps, bool dry, int device);
 bool attach_persist(std::vector<Pass> &ps, bool dry, int device);
 bool attach_occupancy(std::vector<Pass> &ps, bool dry, int device);
+// Lets every tile kernel the passes launch take the device's largest dynamic
+// shared memory (so that no plan made later lowers it under this one).
+bool prepare_tile_fns(const std::vector<Pass> &ps, int device);
 
 // Lazily allocated device staging for host-memory arguments.
 struct Staging {

@@ -268,7 +268,8 @@ mufft_plan_1d *create_1d(int kind, unsigned N, int direction, unsigned flags, un
                            attach_tma(pl->passes, pl->res, dry, pl->device) &&
                            attach_stream(pl->passes, dry, pl->device) &&
                            attach_persist(pl->passes, dry, pl->device) &&
-                           attach_occupancy(pl->passes, dry, pl->device);
+                           attach_occupancy(pl->passes, dry, pl->device) &&
+                           (dry || prepare_tile_fns(pl->passes, pl->device));
         t_opts = prev;
         if (!built) {
             destroy_1d(pl);

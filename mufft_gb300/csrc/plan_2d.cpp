@@ -282,7 +282,8 @@ mufft_plan_2d *create_2d(int kind, unsigned Nx, unsigned Ny, int direction, unsi
         pl->passes.push_back(col);
     }
     if (!attach_stream(pl->passes, dry, pl->device) || !attach_persist(pl->passes, dry, pl->device) ||
-        !attach_occupancy(pl->passes, dry, pl->device)) {
+        !attach_occupancy(pl->passes, dry, pl->device) ||
+        (!dry && !prepare_tile_fns(pl->passes, pl->device))) {
         if (dry)
             delete pl;
         else

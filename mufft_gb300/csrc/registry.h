@@ -7,6 +7,15 @@
 
 namespace mgb {
 
+// A tile kernel compiled for one prologue and epilogue (fft_device.cuh,
+// Flavour): plain inputs, and the named epilogue.
+struct TileFlavours {
+    const void *plain = nullptr;   // plain stores
+    const void *colpow = nullptr;  // four-step twiddle by column powers
+    const void *byrow = nullptr;   // four-step twiddle by grid row
+    const void *r2c = nullptr;     // r2c fix-up, M + 1 bins
+};
+
 struct TileKernel {
     int L;          // transform length
     int R;          // elements per thread
@@ -18,6 +27,7 @@ struct TileKernel {
     size_t smem;    // per CTA
     bool has_thi;   // column pass that takes the four-step twiddle table tw_lo
     size_t smem_ex; // per CTA without the four-step table region (launches with tw_lo == null)
+    TileFlavours fl = {};          // fn for one prologue and epilogue each
     const void *fn_c2r = nullptr;  // row tiles: variant staging c2r fix-up rows in shared memory
 };
 

@@ -93,7 +93,40 @@ static bool uses_c2r_rows(const Pass &p)
 {
     const TileArgs &a = p.a;
     return p.k->fn_c2r && (a.prologue == PRO_C2R || a.prologue == PRO_MUL_C2R) && a.mirror_ldist == 0 &&
-           a.mirror_len == p.k->L && !a.half && a.in_stride == 1;
+           a.mirror_len == p.k->L && !a.half && a.in_stride == 1 && a.epilogue == EPI_PLAIN;
+}
+
+// The kernel of a tile pass: the tile compiled for the pass's prologue and
+// epilogue where there is one, else the tile that decides them at run time.
+static const void *tile_fn(const Pass &p)
+{
+    if (uses_c2r_rows(p))
+        return p.k->fn_c2r;
+    const TileArgs &a = p.a;
+    const void *f = nullptr;
+    if (a.prologue == PRO_PLAIN && !a.half) {
+        if (a.epilogue == EPI_PLAIN)
+            f = p.k->fl.plain;
+        else if (a.epilogue == EPI_R2C)
+            f = p.k->fl.r2c;
+        else if (a.epilogue == EPI_TWIDDLE && a.tw_by_y)
+            f = p.k->fl.byrow;
+        else if (a.epilogue == EPI_TWIDDLE && a.tw_colpow)
+            f = p.k->fl.colpow;
+    }
+    return f ? f : p.k->fn;
+}
+
+bool prepare_tile_fns(const std::vector<Pass> &ps, int device)
+{
+    int limit = 232448;
+    cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+    for (const Pass &p : ps)
+        if (p.type == PASS_TILE && p.k && tile_launch_smem(p) > 48 * 1024 &&
+            !cuda_ok(cudaFuncSetAttribute(tile_fn(p), cudaFuncAttributeMaxDynamicSharedMemorySize, limit),
+                     "cudaFuncSetAttribute(tile)"))
+            return false;
+    return true;
 }
 
 cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream_t st, size_t first, size_t count)
@@ -157,9 +190,7 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
                 cfg.numAttrs = 1;
                 e = cudaLaunchKernelExC(&cfg, p.k->fn, args);
             } else {
-                // c2r fix-up rows staged in shared memory where the tile has that variant
-                e = cudaLaunchKernel(uses_c2r_rows(p) ? p.k->fn_c2r : p.k->fn, p.grid, dim3(p.k->threads), args, smem,
-                                     st);
+                e = cudaLaunchKernel(tile_fn(p), p.grid, dim3(p.k->threads), args, smem, st);
             }
             if (e != cudaSuccess)
                 return e;

@@ -181,7 +181,7 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
     if (flag) {
         // every group is finished: y is complete (L2-coherent loads)
         if (a.inv_c2r_rows)
-            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, true>(a.inv, 0, 0, 0, 0, smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, true, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0, smem);
         else
             tile_body<M, 16, C, 1, ALONG, ALONG, true>(a.inv, 0, 0, 0, 0, smem);
         if (threadIdx.x == 0) {
