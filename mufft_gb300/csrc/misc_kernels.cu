@@ -2,6 +2,7 @@
 // multi-pass transform, the spectral multiply behind mufft_get_convolve_func,
 // and an L2 flush for honest HBM timing.
 #include "fft_device.cuh"
+#include "launch.h"
 #include "misc_kernels.h"
 
 namespace mgb {
@@ -12,6 +13,7 @@ namespace mgb {
 __global__ void r2c_fixup_inplace(float2 *z, const float2 *__restrict__ rtw, long long M,
                                   long long dist, int full)
 {
+    dependent_start();
     float2 *zb = z + (long long)blockIdx.y * dist;
     const long long half = M / 2;
     for (long long k = blockIdx.x * (long long)blockDim.x + threadIdx.x; k <= half;
@@ -56,21 +58,22 @@ __global__ void spectral_multiply(float2 *out, const float2 *__restrict__ a, con
 // The stereo form is the Hermitian part of the correlation spectrum, whose
 // c2r inverse is the real part of the complex correlation.  Signals are
 // summed in index order (deterministic).
-__global__ void adjoint_filter_reduce(float2 *acc, const float2 *__restrict__ g, long long gdist,
-                                      const float2 *__restrict__ a, long long adist, unsigned count,
+__global__ void adjoint_filter_reduce(float2 *acc, const float2 *g, long long gdist,
+                                      const float2 *a, long long adist, unsigned count,
                                       unsigned N, int stereo, float s, int accumulate)
 {
+    dependent_start();
     const unsigned nb = N / 2 + 1;
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
         const unsigned km = (N - k) & (N - 1);
         float2 sum = make_float2(0.f, 0.f);
         for (unsigned i = 0; i < count; i++) {
             const float2 *gi = g + (long long)i * gdist, *ai = a + (long long)i * adist;
-            const float2 gk = gi[k], ak = ai[k];
+            const float2 gk = ld_data(gi + k), ak = ld_data(ai + k);
             sum.x += gk.x * ak.x + gk.y * ak.y;  // G conj(A)
             sum.y += gk.y * ak.x - gk.x * ak.y;
             if (stereo) {
-                const float2 gm = gi[km], am = ai[km];
+                const float2 gm = ld_data(gi + km), am = ld_data(ai + km);
                 sum.x += gm.x * am.x + gm.y * am.y;  // conj(G conj(A)) at N-k
                 sum.y -= gm.y * am.x - gm.x * am.y;
             }
@@ -205,8 +208,8 @@ cudaError_t launch_r2c_fixup_inplace(float2 *z, const float2 *rtw, long long M, 
     unsigned blocks = (unsigned)((work + 255) / 256);
     if (blocks > 4096)
         blocks = 4096;
-    r2c_fixup_inplace<<<dim3(blocks, batch), 256, 0, st>>>(z, rtw, M, dist, full);
-    return cudaGetLastError();
+    void *args[] = {&z, &rtw, &M, &dist, &full};
+    return launch_dependent((const void *)&r2c_fixup_inplace, dim3(blocks, batch), dim3(256), args, 0, st);
 }
 
 cudaError_t launch_spectral_multiply(float2 *out, const float2 *a, const float2 *b, float s,
@@ -229,8 +232,8 @@ cudaError_t launch_adjoint_filter_reduce(float2 *acc, const float2 *g, long long
     unsigned blocks = (nb + 255) / 256;
     if (blocks > 8192)
         blocks = 8192;
-    adjoint_filter_reduce<<<blocks, 256, 0, st>>>(acc, g, gdist, a, adist, count, N, stereo, s, accumulate);
-    return cudaGetLastError();
+    void *args[] = {&acc, &g, &gdist, &a, &adist, &count, &N, &stereo, &s, &accumulate};
+    return launch_dependent((const void *)&adjoint_filter_reduce, dim3(blocks), dim3(256), args, 0, st);
 }
 
 unsigned upols_pitch(unsigned nb) { return (nb + kMacBins - 1) / kMacBins * kMacBins; }

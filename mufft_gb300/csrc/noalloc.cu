@@ -32,6 +32,7 @@
 
 #include "../../include/mufft_gb300.h"
 #include "fft_device.cuh"
+#include "launch.h"
 #include "registry.h"
 
 namespace mgb {
@@ -123,7 +124,7 @@ int set_up(int dev)
 cudaError_t launch(const TileKernel *k, TileArgs &a, unsigned ntrans, cudaStream_t st)
 {
     void *args[] = {&a};
-    return cudaLaunchKernel(k->fn, dim3((ntrans + k->C - 1) / k->C), dim3(k->threads), args,
+    return launch_dependent(k->fn, dim3((ntrans + k->C - 1) / k->C), dim3(k->threads), args,
                             a.tw_lo ? k->smem : k->smem_ex, st);
 }
 

@@ -15,6 +15,7 @@
 #include <cstdio>
 
 #include "host.h"
+#include "launch.h"
 #include "misc_kernels.h"
 
 namespace mgb {
@@ -148,7 +149,7 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
                     int *err = p.tma_err;
                     void *targs[] = {&map, &a, (void *)&tiles_x, &ntiles, &err};
                     const unsigned grid = std::min(ntiles, p.tma_grid);
-                    cudaError_t e = cudaLaunchKernel(p.tk->fn, dim3(grid), dim3(p.tk->threads), targs, p.tk->smem, st);
+                    cudaError_t e = launch_dependent(p.tk->fn, dim3(grid), dim3(p.tk->threads), targs, p.tk->smem, st);
                     if (e != cudaSuccess)
                         return e;
                     continue;
@@ -157,7 +158,7 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
             if (p.pt) {
                 unsigned tiles_x = p.grid.x, ntiles = p.grid.x * p.grid.y;
                 void *pargs[] = {&a, &tiles_x, &ntiles};
-                cudaError_t e = cudaLaunchKernel(p.pt->fn, dim3(std::min(ntiles, p.pt_grid)), dim3(p.pt->threads),
+                cudaError_t e = launch_dependent(p.pt->fn, dim3(std::min(ntiles, p.pt_grid)), dim3(p.pt->threads),
                                                  pargs, tile_launch_smem(p), st);
                 if (e != cudaSuccess)
                     return e;
@@ -166,32 +167,17 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
             if (p.sk) {
                 unsigned ntiles = p.grid.x;
                 void *sargs[] = {&a, &ntiles};
-                cudaError_t e = cudaLaunchKernel(p.sk->fn, dim3(p.sk_grid), dim3(p.sk->threads), sargs, p.sk->smem, st);
+                cudaError_t e = launch_dependent(p.sk->fn, dim3(p.sk_grid), dim3(p.sk->threads), sargs, p.sk->smem, st);
                 if (e != cudaSuccess)
                     return e;
                 continue;
             }
             void *args[] = {&a};
             const size_t smem = tile_launch_smem(p);
-            cudaError_t e;
-            if (p.k->Q > 1) {
-                // one tile per cluster of Q CTAs (distributed shared memory)
-                cudaLaunchConfig_t cfg = {};
-                cudaLaunchAttribute attr[1];
-                cfg.gridDim = dim3(p.grid.x * p.k->Q, p.grid.y, p.grid.z);
-                cfg.blockDim = dim3(p.k->threads);
-                cfg.dynamicSmemBytes = smem;
-                cfg.stream = st;
-                attr[0].id = cudaLaunchAttributeClusterDimension;
-                attr[0].val.clusterDim.x = p.k->Q;
-                attr[0].val.clusterDim.y = 1;
-                attr[0].val.clusterDim.z = 1;
-                cfg.attrs = attr;
-                cfg.numAttrs = 1;
-                e = cudaLaunchKernelExC(&cfg, p.k->fn, args);
-            } else {
-                e = cudaLaunchKernel(tile_fn(p), p.grid, dim3(p.k->threads), args, smem, st);
-            }
+            // one tile per CTA, or per cluster of Q CTAs (distributed shared memory)
+            const unsigned q = (unsigned)p.k->Q;
+            cudaError_t e = launch_dependent(tile_fn(p), dim3(p.grid.x * q, p.grid.y, p.grid.z), dim3(p.k->threads),
+                                             args, smem, st, q);
             if (e != cudaSuccess)
                 return e;
         } else if (p.type == PASS_SPLIT) {
@@ -203,9 +189,9 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
             void *args[] = {&a};
             cudaError_t e =
                 p.sp_engine == 0
-                    ? cudaLaunchKernel(split_umma_kernel(p.sp_stages, p.sp_limbs), dim3(p.sp_grid),
+                    ? launch_dependent(split_umma_kernel(p.sp_stages, p.sp_limbs), dim3(p.sp_grid),
                                        dim3(split_umma_threads()), args, split_umma_smem_bytes(), st)
-                    : cudaLaunchKernel(split_kernel(p.sp_stages, p.sp_limbs), dim3(p.sp_grid), dim3(kSplitThreads),
+                    : launch_dependent(split_kernel(p.sp_stages, p.sp_limbs), dim3(p.sp_grid), dim3(kSplitThreads),
                                        args, split_smem_bytes(), st);
             if (e != cudaSuccess)
                 return e;

@@ -93,13 +93,14 @@ __global__ void __launch_bounds__(kSplitThreads, 2) split_tc_fft(const SplitArgs
                 af[l][m][r] = __ldg(&a.afrag[((l * 3 + m) * 32 + lane) * 4 + r]);
     for (int i = threadIdx.x; i < 512; i += kSplitThreads)
         t1[i] = __ldg(&a.tw[i]);
+    dependent_start();  // the tables are the plan's; what follows reads the caller's input
 
 #pragma unroll 4
     for (int e = threadIdx.x; e < kSplitPoints; e += kSplitThreads) {
         const int t = e / N, n = e % N;
         float2 v = make_float2(0.f, 0.f);
         if (tr0 + t < a.ntrans)
-            v = __ldg(&a.in[(tr0 + t) * a.in_dist + n]);
+            v = ld_data(&a.in[(tr0 + t) * a.in_dist + n]);
         if (a.conj)
             v.y = -v.y;
         src[spad(e)] = v;

@@ -208,6 +208,9 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
             asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar0 + 8 * b), "r"(1));
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    // the tables above are the plan's; what follows reads the caller's input.
+    // Before the allocation: a CTA that holds TMEM waits for no other kernel
+    dependent_start();
     if (warp == 0) {
         asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
                      "r"(kTmemCols));
@@ -249,7 +252,7 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
                 const int t = e / N, n = e % N;
                 float2 v = make_float2(0.f, 0.f);
                 if (tr0 + t < a.ntrans)
-                    v = __ldg(&a.in[(tr0 + t) * a.in_dist + n]);
+                    v = ld_data(&a.in[(tr0 + t) * a.in_dist + n]);
                 if (a.conj)
                     v.y = -v.y;
                 X[upad(e)] = v;

@@ -21,6 +21,7 @@
 //   tickets[0] = k, [1] groups finished, [2] = k + 1 once the spectrum of
 //   block k is out, [3 + x] range CTAs done with group x.
 #include "fft_device.cuh"
+#include "launch.h"
 #include "stream_conv.h"
 
 namespace mgb {
@@ -94,6 +95,7 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
     __shared__ unsigned flag;
     constexpr int C = 4096 / M;
     static_assert(C * (M / 16) == 256, "256-thread row tile");
+    dependent_start();
     const unsigned k = *(volatile unsigned *)&a.tickets[0];
     const unsigned cur = k % a.P;
     const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
@@ -119,7 +121,7 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
 #pragma unroll 8
     for (unsigned p = p0 + w; p < p1; p += kWarps) {
         const unsigned slot = cur >= p ? cur - p : cur + a.P - p;  // block k - p
-        cmac2(acc, __ldg((const float4 *)&a.fdl[(size_t)slot * a.pitch + b]),
+        cmac2(acc, ld_data4((const float4 *)&a.fdl[(size_t)slot * a.pitch + b]),
               __ldg((const float4 *)&a.h[(size_t)p * a.pitch + b]));
     }
     red[w][lane] = acc;
@@ -233,7 +235,7 @@ cudaError_t launch_upols_block(int M, const UpolsBlockArgs &a, cudaStream_t st)
     UpolsBlockArgs args = a;
     void *params[] = {&args};
     const unsigned grid = 1 + a.groups * a.G;
-    return cudaLaunchKernel(fn, dim3(grid), dim3(256), params, upols_block_smem(M), st);
+    return launch_dependent(fn, dim3(grid), dim3(256), params, upols_block_smem(M), st);
 }
 
 }  // namespace mgb

@@ -28,6 +28,7 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, 1>(), tile_min_blocks<L,
     tile_fft_persist(const TileArgs a, const unsigned tiles_x, const unsigned ntiles)
 {
     extern __shared__ float2 smem[];
+    dependent_start();
     for (unsigned t = blockIdx.x; t < ntiles; t += gridDim.x) {
         const unsigned tx = t % tiles_x, z = t / tiles_x;
         long long ioff, ooff;

@@ -20,6 +20,7 @@ template <int L, int R, int C>
 __global__ void __launch_bounds__(tile_threads<L, R, C, 1>()) tile_fft_stream(const TileArgs a, const unsigned ntiles)
 {
     extern __shared__ float2 smem[];
+    dependent_start();
     constexpr int TL = Tile<L, R, 1>::TL;
     unsigned t = blockIdx.x;
     if (t >= ntiles)

@@ -69,6 +69,7 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, 1>(), 2)
                  const unsigned ntiles, int *err)
 {
     extern __shared__ __align__(1024) unsigned char sm[];
+    dependent_start();
     constexpr size_t BUF = tma_buf_bytes<L, R, C>();
     float2 *ex = (float2 *)(sm + NBUF * BUF);
     unsigned long long *bars = (unsigned long long *)(sm + NBUF * BUF + tma_region_bytes<L, R, C>());
