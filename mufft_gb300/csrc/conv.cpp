@@ -26,6 +26,8 @@ struct mufft_plan_conv {
     float2 *adj_spec = nullptr;              // spectra of the gradients
     size_t adj_spec_bytes = 0;
     float2 *adj_acc = nullptr;               // N/2 + 1 bins of the filter gradient
+    void *adj_part = nullptr;                // rows of partial sums of the reduction over signals
+    size_t adj_part_bytes = 0;
     // batched forms (mufft_gb_execute_conv_output_batched, mufft_gb_conv_adjoint):
     // plans over a chunk of signals and over the ragged last chunk
     struct BatchPlan {
@@ -148,6 +150,7 @@ void mufft_free_plan_conv(mufft_plan_conv *plan)
         DeviceGuard g(plan->device);
         cudaFree(plan->adj_spec);
         cudaFree(plan->adj_acc);
+        cudaFree(plan->adj_part);
     }
     delete plan;
 }
@@ -181,6 +184,21 @@ bool conv_adj_spec(mufft_plan_conv *c, size_t bytes)
         return false;
     c->adj_spec_bytes = bytes;
     return true;
+}
+
+// Sums the gradients' spectra of `n` signals (adj_spec) against their first
+// spectra into the filter gradient's bins.
+bool conv_reduce(mufft_plan_conv *c, const float2 *first, size_t dist, unsigned n, bool accumulate, cudaStream_t st)
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    const unsigned rows = adjoint_reduce_rows(c->N, n, sms);
+    if (rows > 1 && !ensure(c->adj_part, c->adj_part_bytes, (size_t)rows * (c->N / 2 + 1) * sizeof(float2)))
+        return false;
+    return cuda_ok(launch_adjoint_filter_reduce(c->adj_acc, (float2 *)c->adj_part, rows, c->adj_spec,
+                                                (long long)conv_bins(c), first, (long long)dist, n, c->N,
+                                                conv_stereo(c) ? 1 : 0, 1.0f / (float)c->N, accumulate ? 1 : 0, st),
+                   "adjoint reduce");
 }
 
 }  // namespace
@@ -280,10 +298,7 @@ int mufft_gb_conv_adjoint_filter(mufft_plan_conv *plan, float *grad_filter, cons
                     return rc;
             }
         }
-        if (!cuda_ok(launch_adjoint_filter_reduce(plan->adj_acc, plan->adj_spec, (long long)bins,
-                                                  A + b0 * spectrum_dist, (long long)spectrum_dist, (unsigned)n,
-                                                  N, stereo ? 1 : 0, 1.0f / (float)N, b0 > 0 ? 1 : 0, st),
-                     "adjoint reduce"))
+        if (!conv_reduce(plan, A + b0 * spectrum_dist, spectrum_dist, (unsigned)n, b0 > 0, st))
             return t_err;
     }
     return exec_1d(plan->adj_c2r, grad_filter, plan->adj_acc, nullptr, st, false);
@@ -420,11 +435,7 @@ int mufft_gb_conv_adjoint(mufft_plan_conv *plan, float *grad_filter, void *grad_
         int rc = exec_1d(fwd, plan->adj_spec, (const char *)grad_outputs + b0 * output_dist * elem, nullptr, st, false);
         if (rc != MUFFT_GB_OK)
             return rc;
-        if (grad_filter &&
-            !cuda_ok(launch_adjoint_filter_reduce(plan->adj_acc, plan->adj_spec, (long long)bins,
-                                                  A + b0 * spectrum_dist, (long long)spectrum_dist, (unsigned)n, N,
-                                                  stereo ? 1 : 0, 1.0f / (float)N, b0 > 0 ? 1 : 0, st),
-                     "adjoint reduce"))
+        if (grad_filter && !conv_reduce(plan, A + b0 * spectrum_dist, spectrum_dist, (unsigned)n, b0 > 0, st))
             return t_err;
         if (grad_inputs) {
             mufft_plan_1d *inv = conv_batch_plan(plan->inv_b[w], stereo ? K_C2C : K_C2R, N, MUFFT_INVERSE,

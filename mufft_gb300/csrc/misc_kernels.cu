@@ -1,6 +1,8 @@
 // Small element-wise kernels: the in-place real-to-complex fix-up used after a
 // multi-pass transform, the spectral multiply behind mufft_get_convolve_func,
 // and an L2 flush for honest HBM timing.
+#include <algorithm>
+
 #include "fft_device.cuh"
 #include "launch.h"
 #include "misc_kernels.h"
@@ -56,19 +58,27 @@ __global__ void spectral_multiply(float2 *out, const float2 *__restrict__ a, con
 //   stereo (full c2c spectra):     acc[k] (+)= s/2 * sum_i (G_i[k] conj(A_i[k])
 //                                               + conj(G_i[N-k] conj(A_i[N-k])))
 // The stereo form is the Hermitian part of the correlation spectrum, whose
-// c2r inverse is the real part of the complex correlation.  Signals are
-// summed in index order (deterministic).
-__global__ void adjoint_filter_reduce(float2 *acc, const float2 *g, long long gdist,
-                                      const float2 *a, long long adist, unsigned count,
-                                      unsigned N, int stereo, float s, int accumulate)
+// c2r inverse is the real part of the complex correlation.
+// Few bins and many signals would leave the GPU idle with one thread a bin, so
+// grid row y takes signals y*count/Y .. (y+1)*count/Y - 1 and, for Y > 1,
+// writes its sum to row y of `part`; adjoint_filter_sum adds the rows in order
+// (deterministic).  700 signals of 8192: 576 us as one row, 8 us as 38.
+__global__ void __launch_bounds__(256) adjoint_filter_reduce(float2 *acc, float2 *part, const float2 *g,
+                                                             long long gdist, const float2 *a, long long adist,
+                                                             unsigned count, unsigned N, int stereo, float s,
+                                                             int accumulate)
 {
     dependent_start();
     const unsigned nb = N / 2 + 1;
+    const unsigned Y = gridDim.y, y = blockIdx.y;
+    const unsigned i0 = (unsigned)((unsigned long long)count * y / Y),
+                   i1 = (unsigned)((unsigned long long)count * (y + 1) / Y);
     for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
         const unsigned km = (N - k) & (N - 1);
         float2 sum = make_float2(0.f, 0.f);
-        for (unsigned i = 0; i < count; i++) {
-            const float2 *gi = g + (long long)i * gdist, *ai = a + (long long)i * adist;
+        const float2 *gi = g + (long long)i0 * gdist, *ai = a + (long long)i0 * adist;
+#pragma unroll 4
+        for (unsigned i = i0; i < i1; i++) {
             const float2 gk = ld_data(gi + k), ak = ld_data(ai + k);
             sum.x += gk.x * ak.x + gk.y * ak.y;  // G conj(A)
             sum.y += gk.y * ak.x - gk.x * ak.y;
@@ -77,6 +87,12 @@ __global__ void adjoint_filter_reduce(float2 *acc, const float2 *g, long long gd
                 sum.x += gm.x * am.x + gm.y * am.y;  // conj(G conj(A)) at N-k
                 sum.y -= gm.y * am.x - gm.x * am.y;
             }
+            gi += gdist;
+            ai += adist;
+        }
+        if (Y > 1) {
+            part[(size_t)y * nb + k] = sum;
+            continue;
         }
         const float f = stereo ? 0.5f * s : s;
         float2 r = make_float2(sum.x * f, sum.y * f);
@@ -84,6 +100,23 @@ __global__ void adjoint_filter_reduce(float2 *acc, const float2 *g, long long gd
             r.x += acc[k].x;
             r.y += acc[k].y;
         }
+        acc[k] = r;
+    }
+}
+
+// acc[k] (+)= f * (row 0 + row 1 + ... of part), in row order.
+__global__ void __launch_bounds__(256) adjoint_filter_sum(float2 *acc, const float2 *part, unsigned rows, unsigned nb,
+                                                          float f, int accumulate)
+{
+    dependent_start();
+    for (unsigned k = blockIdx.x * blockDim.x + threadIdx.x; k < nb; k += gridDim.x * blockDim.x) {
+        float2 sum = make_float2(0.f, 0.f);
+#pragma unroll 8
+        for (unsigned y = 0; y < rows; y++)
+            sum = cadd(sum, ld_data(part + (size_t)y * nb + k));
+        float2 r = cscale(sum, f);
+        if (accumulate)
+            r = cadd(r, acc[k]);
         acc[k] = r;
     }
 }
@@ -224,16 +257,31 @@ cudaError_t launch_spectral_multiply(float2 *out, const float2 *a, const float2 
     return cudaGetLastError();
 }
 
-cudaError_t launch_adjoint_filter_reduce(float2 *acc, const float2 *g, long long gdist, const float2 *a,
-                                         long long adist, unsigned count, unsigned N, int stereo, float s,
-                                         int accumulate, cudaStream_t st)
+// Rows of signals that fill the GPU: four 256-thread CTAs an SM, at least
+// eight signals a row.
+unsigned adjoint_reduce_rows(unsigned N, unsigned count, int sms)
 {
+    const unsigned long long want = 4ull * 256 * (unsigned)(sms > 0 ? sms : 152);
     const unsigned nb = N / 2 + 1;
+    const unsigned rows = (unsigned)std::min<unsigned long long>((want + nb - 1) / nb, 64);
+    return std::max(1u, std::min(rows, count / 8));
+}
+
+cudaError_t launch_adjoint_filter_reduce(float2 *acc, float2 *part, unsigned rows, const float2 *g, long long gdist,
+                                         const float2 *a, long long adist, unsigned count, unsigned N, int stereo,
+                                         float s, int accumulate, cudaStream_t st)
+{
+    unsigned nb = N / 2 + 1;
     unsigned blocks = (nb + 255) / 256;
     if (blocks > 8192)
         blocks = 8192;
-    void *args[] = {&acc, &g, &gdist, &a, &adist, &count, &N, &stereo, &s, &accumulate};
-    return launch_dependent((const void *)&adjoint_filter_reduce, dim3(blocks), dim3(256), args, 0, st);
+    void *args[] = {&acc, &part, &g, &gdist, &a, &adist, &count, &N, &stereo, &s, &accumulate};
+    cudaError_t e = launch_dependent((const void *)&adjoint_filter_reduce, dim3(blocks, rows), dim3(256), args, 0, st);
+    if (e != cudaSuccess || rows == 1)
+        return e;
+    float f = stereo ? 0.5f * s : s;
+    void *sargs[] = {&acc, &part, &rows, &nb, &f, &accumulate};
+    return launch_dependent((const void *)&adjoint_filter_sum, dim3(blocks), dim3(256), sargs, 0, st);
 }
 
 unsigned upols_pitch(unsigned nb) { return (nb + kMacBins - 1) / kMacBins * kMacBins; }

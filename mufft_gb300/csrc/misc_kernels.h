@@ -9,9 +9,12 @@ cudaError_t launch_r2c_fixup_inplace(float2 *z, const float2 *rtw, long long M, 
                                      unsigned batch, int full, cudaStream_t st);
 cudaError_t launch_spectral_multiply(float2 *out, const float2 *a, const float2 *b, float s,
                                      unsigned long long n, cudaStream_t st);
-cudaError_t launch_adjoint_filter_reduce(float2 *acc, const float2 *g, long long gdist, const float2 *a,
-                                         long long adist, unsigned count, unsigned N, int stereo, float s,
-                                         int accumulate, cudaStream_t st);
+// Reduction rows for `count` signals, and the reduction: part holds rows x
+// (N/2 + 1) bins where rows > 1.
+unsigned adjoint_reduce_rows(unsigned N, unsigned count, int sms);
+cudaError_t launch_adjoint_filter_reduce(float2 *acc, float2 *part, unsigned rows, const float2 *g, long long gdist,
+                                         const float2 *a, long long adist, unsigned count, unsigned N, int stereo,
+                                         float s, int accumulate, cudaStream_t st);
 // Partitioned overlap-save multiply-accumulate over (64-bin groups) x G
 // partition ranges.  fdl and h: P rows of upols_pitch(nb) bins (pad bins
 // zero); part: G rows of that pitch; tickets: 2 + upols_groups(nb) counters,
