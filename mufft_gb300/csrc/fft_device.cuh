@@ -150,20 +150,67 @@ template <> struct Dft<16> {
     }
 };
 
+// 32 = 16 x 2: DFT-16 over the even and the odd samples, the odd one's outputs
+// times W32^k, then sums and differences.
+template <> struct Dft<32> {
+    __device__ __forceinline__ static void run(float2 *v)
+    {
+        float2 e[16], o[16];
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            e[k] = v[2 * k];
+            o[k] = v[2 * k + 1];
+        }
+        Dft<16>::run(e);
+        Dft<16>::run(o);
+        // cos and sin of k*pi/16
+        constexpr float C[8] = {1.f,
+                                0.98078528040323044913f,
+                                kCos8,
+                                0.83146961230254523708f,
+                                kRsqrt2,
+                                0.55557023301960222474f,
+                                kSin8,
+                                0.19509032201612826785f};
+#pragma unroll
+        for (int k = 0; k < 16; k++) {
+            float2 t = o[k];
+            if (k == 4)
+                t = mul_w8_1(t);
+            else if (k == 8)
+                t = mul_neg_i(t);
+            else if (k == 12)
+                t = mul_w8_3(t);
+            else if (k != 0)
+                t = cmul(t, k < 8 ? make_float2(C[k], -C[(8 - k) & 7]) : make_float2(-C[(16 - k) & 7], -C[k - 8]));
+            v[k] = cadd(e[k], t);
+            v[k + 16] = csub(e[k], t);
+        }
+    }
+};
+
 // ------------------------------------------------------------- schedule
 
 constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
 
 // Stage plan of a length-L transform whose threads own R elements each:
-// radix-16 stages, then one smaller stage for the leftover factor.
+// radix-16 stages, then one smaller stage for the leftover factor; threads of
+// 32 elements take radix-32 stages last where that saves a stage (and its
+// exchange through shared memory): 512 = 16 x 32,
+// 8192 = 16 x 16 x 32, 16384 = 16 x 32 x 32.
 template <int L, int R> struct Sched {
     static_assert(L >= 2 && (L & (L - 1)) == 0, "power of two");
     static_assert(R <= L && L % R == 0, "R divides L");
     static constexpr int LOG = ilog2c(L);
-    static constexpr int NFULL = L < 16 ? 0 : LOG / 4;
-    static constexpr int REMB = L < 16 ? LOG : LOG % 4;
-    static constexpr int NST = NFULL + (REMB ? 1 : 0);
-    __host__ __device__ static constexpr int radix(int s) { return s < NFULL ? 16 : (1 << REMB); }
+    static constexpr bool WIDE = R == 32 && (LOG + 4) / 5 < (LOG + 3) / 4 && LOG <= 14 && LOG != 10;
+    static constexpr int N32 = WIDE ? LOG - 4 * ((LOG + 4) / 5) : 0;
+    static constexpr int NFULL = WIDE ? (LOG + 4) / 5 - N32 : (L < 16 ? 0 : LOG / 4);
+    static constexpr int REMB = WIDE ? 0 : (L < 16 ? LOG : LOG % 4);
+    static constexpr int NST = NFULL + N32 + (REMB ? 1 : 0);
+    __host__ __device__ static constexpr int radix(int s)
+    {
+        return s < NFULL ? 16 : (s < NFULL + N32 ? 32 : (1 << REMB));
+    }
     __host__ __device__ static constexpr int pbefore(int s)
     {
         int p = 1;
@@ -258,9 +305,10 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, con
         if constexpr (p > 1) {
             const int i = j * TT::B(s) + tl + TT::TL * u;
             const int k = i & (p - 1);
-            const float4 *e = reinterpret_cast<const float4 *>(tw + stage_table_base(r, p) + 4 * k);
+            const float4 *e = reinterpret_cast<const float4 *>(
+                r == 32 ? tw + stage32_base(p) + 8 * k : tw + stage_table_base(r, p) + 4 * k);
             const float4 a = __ldg(e);
-            float2 w[16];
+            float2 w[r < 16 ? 16 : r];
             w[1] = make_float2(a.x, a.y);
             w[2] = make_float2(a.z, a.w);
             if constexpr (r > 4) {
@@ -268,25 +316,27 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, con
                 w[4] = make_float2(b.x, b.y);
                 w[8] = make_float2(b.z, b.w);
             }
+            if constexpr (r > 16)
+                w[16] = __ldg(reinterpret_cast<const float2 *>(e + 2));
             if constexpr (BASE) {
                 // base * W^(mk): base, then each power from one half as long
                 float2 z[r];
                 z[0] = base;
 #pragma unroll
                 for (int m = 1; m < r; m++) {
-                    const int hi = m >= 8 ? 8 : (m >= 4 ? 4 : (m >= 2 ? 2 : 1));
+                    const int hi = m >= 16 ? 16 : (m >= 8 ? 8 : (m >= 4 ? 4 : (m >= 2 ? 2 : 1)));
                     z[m] = cmul(z[m - hi], w[hi]);
                 }
 #pragma unroll
                 for (int m = 0; m < r; m++)
                     v[u * r + m] = cmul(v[u * r + m], z[m]);
             } else {
-                // remaining powers: at most three rounded products deep
+                // remaining powers: at most three rounded products deep (four for radix 32)
 #pragma unroll
                 for (int m = 3; m < r; m++) {
-                    if (m == 4 || m == 8)
+                    if (m == 4 || m == 8 || m == 16)
                         continue;
-                    const int hi = m >= 8 ? 8 : (m >= 4 ? 4 : 2);
+                    const int hi = m >= 16 ? 16 : (m >= 8 ? 8 : (m >= 4 ? 4 : 2));
                     w[m] = cmul(w[m - hi], w[hi]);
                 }
 #pragma unroll
@@ -790,11 +840,13 @@ __device__ __forceinline__ void run_stages(float2 (&v)[R], int j, int &c, int &t
 }
 
 // Threads of one CTA, and the CTAs per SM the register budget is sized for:
-// 16-element tiles are held to 64 registers so that 2048 threads fit.
+// 16-element tiles are held to 64 registers so that 1024 threads fit, 32-element
+// ones to 128 (512 threads).
 template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_threads() { return C * (L / (R * Q)); }
 template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_min_blocks()
 {
-    return R <= 16 ? (tile_threads<L, R, C, Q>() >= 1024 ? 1 : 1024 / tile_threads<L, R, C, Q>()) : 1;
+    constexpr int most = R <= 16 ? 1024 : 512;  // 64, or 128 registers a thread
+    return tile_threads<L, R, C, Q>() >= most ? 1 : most / tile_threads<L, R, C, Q>();
 }
 
 // One tile of C transforms: load, all stages, store.  `tile` selects the

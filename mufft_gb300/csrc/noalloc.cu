@@ -50,12 +50,21 @@ __global__ void noalloc_fill_twiddles(float2 *t)
 {
     const int n = kStageTableFloat2;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
-        const int per_radix = kStageTableK * 4;
-        const int ri = idx / per_radix;
-        const int kk = (idx % per_radix) / 4, e = idx % 4;
-        const int r = 2 << ri;
-        const int p = kk < 16 ? 16 : (kk < 272 ? 256 : 4096);
-        const int k = kk - stage_p_offset(p);
+        int r, p, k, e;
+        if (idx < kStage32Begin) {
+            const int per_radix = kStageTableK * 4;
+            const int ri = idx / per_radix;
+            const int kk = (idx % per_radix) / 4;
+            e = idx % 4;
+            r = 2 << ri;
+            p = kk < 16 ? 16 : (kk < 272 ? 256 : 4096);
+            k = kk - stage_p_offset(p);
+        } else {
+            e = (idx - kStage32Begin) % 8;
+            r = 32;
+            p = idx < stage32_base(256) ? 16 : idx < stage32_base(512) ? 256 : 512;
+            k = (idx - stage32_base(p)) / 8;
+        }
         const long long rp = (long long)r * p;
         const long long m = ((long long)(1 << e) * k) % rp;
         double s, c;

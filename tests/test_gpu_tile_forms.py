@@ -72,3 +72,27 @@ def test_column_twiddle_forms(gpu, torch, mode):
     ref = np.fft.fft(x.astype(np.complex128), axis=1)
     got = _run(gpu, torch, 0, N, K.FORWARD, 0, x, (B, N), gpu.options(twiddle_table=mode))
     assert rel_l2(got, ref) <= 2.0 ** -23 * 17
+
+
+@pytest.mark.parametrize("tile", [(512, 0, 0, 16, 32, 1), (512, 0, 0, 8, 16, 1), (8192, 0, 0, 1, 32, 1),
+                                  (8192, 0, 0, 1, 16, 1), (16384, 0, 0, 1, 32, 1), (16384, 0, 0, 1, 16, 1)])
+@pytest.mark.parametrize("kind", [0, 1, 2])
+def test_wide_radix_rows(gpu, torch, tile, kind):
+    """Row tiles of 16 and of 32 elements a thread (radix-32 stages), every kind."""
+    L, B = tile[0], 17
+    N = L if kind == 0 else 2 * L
+    lg = N.bit_length() - 1
+    opts = gpu.options(tiles=[tile])
+    x = signals.complex_uniform(84000 + N + kind, B * N).reshape(B, N)
+    if kind == 0:
+        got = _run(gpu, torch, 0, N, K.INVERSE, 0, x, (B, N), opts)
+        assert rel_l2(got, np.fft.ifft(x.astype(np.complex128), axis=1) * N) <= 2.0 ** -23 * lg
+        return
+    xr = np.ascontiguousarray(x.real)
+    X = np.fft.rfft(xr.astype(np.float64), axis=1)
+    if kind == 1:
+        assert rel_l2(_run(gpu, torch, 1, N, K.FORWARD, 0, xr, (B, N // 2 + 1), opts), X) <= 2.0 ** -23 * lg
+        return
+    Xs = X.astype(np.complex64)
+    back = _run(gpu, torch, 2, N, K.INVERSE, 0, Xs, (B, N // 2), opts).view(np.float32)
+    assert rel_l2(back, np.fft.irfft(Xs.astype(np.complex128), axis=1) * N) <= 2.0 ** -23 * lg
