@@ -27,15 +27,17 @@ __host__ __device__ constexpr int stage_table_base(int r, int p)
 {
     return (stage_radix_index(r) * kStageTableK + stage_p_offset(p)) * 4;
 }
-// Radix-32 stages (p in {16, 256, 512}) follow, eight float2 for each k:
-// W^k, W^2k, W^4k, W^8k, W^16k and three unused.
+// Radix-32 stages (p in {16, 32, 256, 512}) follow, eight float2 for each k:
+// W^(e*k) for the exponents e below (the last one unused), so that every power
+// is a product of at most three.
 constexpr int kStage32Begin = 4 * kStageTableK * 4;
-constexpr int kStage32Sizes[3] = {16, 256, 512};
+constexpr int kStage32Exps[8] = {1, 2, 4, 8, 3, 12, 16, 0};
+constexpr int kStage32Sizes[4] = {16, 32, 256, 512};
 __host__ __device__ constexpr int stage32_base(int p)
 {
-    return kStage32Begin + 8 * (p == 16 ? 0 : p == 256 ? 16 : 272);
+    return kStage32Begin + 8 * (p == 16 ? 0 : p == 32 ? 16 : p == 256 ? 48 : 304);
 }
-constexpr int kStageTableFloat2 = kStage32Begin + 8 * (16 + 256 + 512);
+constexpr int kStageTableFloat2 = kStage32Begin + 8 * (16 + 32 + 256 + 512);
 
 // Thread-to-work decomposition of a CTA: which index runs fastest across
 // consecutive threads.  ALONG: consecutive threads walk along one transform

@@ -202,7 +202,7 @@ template <int L, int R> struct Sched {
     static_assert(L >= 2 && (L & (L - 1)) == 0, "power of two");
     static_assert(R <= L && L % R == 0, "R divides L");
     static constexpr int LOG = ilog2c(L);
-    static constexpr bool WIDE = R == 32 && (LOG + 4) / 5 < (LOG + 3) / 4 && LOG <= 14 && LOG != 10;
+    static constexpr bool WIDE = R == 32 && (LOG + 4) / 5 < (LOG + 3) / 4 && LOG <= 14;
     static constexpr int N32 = WIDE ? LOG - 4 * ((LOG + 4) / 5) : 0;
     static constexpr int NFULL = WIDE ? (LOG + 4) / 5 - N32 : (L < 16 ? 0 : LOG / 4);
     static constexpr int REMB = WIDE ? 0 : (L < 16 ? LOG : LOG % 4);
@@ -211,6 +211,8 @@ template <int L, int R> struct Sched {
     {
         return s < NFULL ? 16 : (s < NFULL + N32 ? 32 : (1 << REMB));
     }
+    // padding of the exchange slices: one slot every 2^PS positions
+    static constexpr int PS = (WIDE && NFULL == 0) ? 5 : 4, PN = 1 << PS;
     __host__ __device__ static constexpr int pbefore(int s)
     {
         int p = 1;
@@ -249,12 +251,13 @@ template <int L, int R, int Q> struct Tile {
 // banks; an extra offset makes the slice stride ≡ 16/C (mod 16) so that the
 // 16 lanes of a half-warp walking ACROSS C transforms hit 16 distinct bank
 // pairs (64-bit accesses are served per half-warp).
-template <int LQ, int C, bool ACROSS_USED>
+// (A transform whose first stage is radix 32 is padded every 32: PS 5.)
+template <int LQ, int C, bool ACROSS_USED, int PS = 4>
 __host__ __device__ constexpr int region_stride()
 {
     if (LQ < 16)
         return LQ;
-    int base = LQ + LQ / 16;
+    int base = LQ + (LQ >> PS);
     if (!ACROSS_USED || C < 2)
         return base;
     int want = C >= 16 ? 1 : 16 / C;
@@ -262,7 +265,7 @@ __host__ __device__ constexpr int region_stride()
     return base + ((want - have + 16) % 16);
 }
 
-__device__ __forceinline__ int padpos(int pos) { return pos + (pos >> 4); }
+template <int PS> __device__ __forceinline__ int padpos(int pos) { return pos + (pos >> PS); }
 
 template <int MAP, int C, int T>
 __device__ __forceinline__ void split_tid(int tid, int &c, int &t)
@@ -286,6 +289,15 @@ __device__ __forceinline__ void tile_sync()
 }
 
 // ---------------------------------------------------------------- stages
+
+// The largest power of the table's that is at most m and leaves a smaller one
+// in m - it: 1, 2, 4, 8 -- and for radix 32 also 3, 12 and 16, m = 16a + 4b + c.
+template <int r> __host__ __device__ constexpr int twiddle_top(int m)
+{
+    if (r == 32)
+        return m >= 16 ? 16 : (m >= 4 ? m & ~3 : m);
+    return m >= 8 ? 8 : (m >= 4 ? 4 : (m >= 2 ? 2 : 1));
+}
 
 // Twiddle multiply and DFT of stage s on the thread's R registers.
 // Register u*r + m holds input m of butterfly i = j*B + tl + TL*u.
@@ -316,28 +328,31 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, con
                 w[4] = make_float2(b.x, b.y);
                 w[8] = make_float2(b.z, b.w);
             }
-            if constexpr (r > 16)
-                w[16] = __ldg(reinterpret_cast<const float2 *>(e + 2));
+            if constexpr (r == 32) {
+                const float4 c = __ldg(e + 2), d = __ldg(e + 3);
+                w[3] = make_float2(c.x, c.y);
+                w[12] = make_float2(c.z, c.w);
+                w[16] = make_float2(d.x, d.y);
+            }
             if constexpr (BASE) {
-                // base * W^(mk): base, then each power from one half as long
+                // base * W^(mk): base, then each power times one of the table's
                 float2 z[r];
                 z[0] = base;
 #pragma unroll
                 for (int m = 1; m < r; m++) {
-                    const int hi = m >= 16 ? 16 : (m >= 8 ? 8 : (m >= 4 ? 4 : (m >= 2 ? 2 : 1)));
+                    const int hi = twiddle_top<r>(m);
                     z[m] = cmul(z[m - hi], w[hi]);
                 }
 #pragma unroll
                 for (int m = 0; m < r; m++)
                     v[u * r + m] = cmul(v[u * r + m], z[m]);
             } else {
-                // remaining powers: at most three rounded products deep (four for radix 32)
+                // remaining powers: at most three rounded products deep (two for radix 32)
 #pragma unroll
                 for (int m = 3; m < r; m++) {
-                    if (m == 4 || m == 8 || m == 16)
-                        continue;
-                    const int hi = m >= 16 ? 16 : (m >= 8 ? 8 : (m >= 4 ? 4 : 2));
-                    w[m] = cmul(w[m - hi], w[hi]);
+                    const int hi = twiddle_top<r>(m);
+                    if (hi != m)
+                        w[m] = cmul(w[m - hi], w[hi]);
                 }
 #pragma unroll
                 for (int m = 1; m < r; m++)
@@ -350,25 +365,26 @@ __device__ __forceinline__ void stage_compute(float2 (&v)[R], int j, int tl, con
 
 // Store the outputs of stage s into the CTA's own slice (local offset
 // pos - j*LQ).  Output m of butterfly i goes to (i - k)*r + k + m*p; when p
-// is a multiple of 16 the padded address is padpos(base) + m*(p + p/16), and
-// for p == 1, r == 16 it is 17*(i - j*LQ/16) + m: a base plus constants.
+// is a multiple of PN (16, or 32) the padded address is padpos(base) +
+// m*(p + p/PN), and for p == 1, r == PN it is (PN + 1)*(i - j*LQ/PN) + m: a base
+// plus constants.
 template <int L, int R, int Q, int s>
 __device__ __forceinline__ void stage_write(float2 *region, const float2 (&v)[R], int j, int tl)
 {
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
-    constexpr int r = S::radix(s), p = S::pbefore(s), NB = R / r;
+    constexpr int r = S::radix(s), p = S::pbefore(s), NB = R / r, PS = S::PS, PN = S::PN;
 #pragma unroll
     for (int u = 0; u < NB; u++) {
         const int i = j * TT::B(s) + tl + TT::TL * u;
-        if constexpr (p % 16 == 0) {
+        if constexpr (p % PN == 0) {
             const int k = i & (p - 1);
-            float2 *b = region + padpos((i - k) * r + k - j * TT::LQ);
+            float2 *b = region + padpos<PS>((i - k) * r + k - j * TT::LQ);
 #pragma unroll
             for (int m = 0; m < r; m++)
-                b[m * (p + p / 16)] = v[u * r + m];
-        } else if constexpr (p == 1 && r == 16) {
-            float2 *b = region + 17 * (i - j * (TT::LQ / 16));
+                b[m * (p + p / PN)] = v[u * r + m];
+        } else if constexpr (p == 1 && r == PN) {
+            float2 *b = region + (PN + 1) * (i - j * (TT::LQ / PN));
 #pragma unroll
             for (int m = 0; m < r; m++)
                 b[m] = v[u * r + m];
@@ -377,7 +393,7 @@ __device__ __forceinline__ void stage_write(float2 *region, const float2 (&v)[R]
             const int base = (i - k) * r + k - j * TT::LQ;
 #pragma unroll
             for (int m = 0; m < r; m++)
-                region[padpos(base + m * p)] = v[u * r + m];
+                region[padpos<PS>(base + m * p)] = v[u * r + m];
         }
     }
 }
@@ -390,26 +406,26 @@ __device__ __forceinline__ void stage_read(float2 *region, float2 (&v)[R], int j
 {
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
-    constexpr int r = S::radix(s), NB = R / r, B = TT::B(s), TL = TT::TL;
-    if constexpr (Q == 1 && TL % 16 == 0 && B % 16 == 0) {
-        const float2 *b = region + padpos(tl);
+    constexpr int r = S::radix(s), NB = R / r, B = TT::B(s), TL = TT::TL, PS = S::PS, PN = S::PN;
+    if constexpr (Q == 1 && TL % PN == 0 && B % PN == 0) {
+        const float2 *b = region + padpos<PS>(tl);
 #pragma unroll
         for (int u = 0; u < NB; u++)
 #pragma unroll
             for (int m = 0; m < r; m++)
-                v[u * r + m] = b[(B * m + TL * u) / 16 * 17];
-    } else if constexpr (TL % 16 == 0 && B % 16 == 0 && r % Q == 0) {
+                v[u * r + m] = b[(B * m + TL * u) / PN * (PN + 1)];
+    } else if constexpr (TL % PN == 0 && B % PN == 0 && r % Q == 0) {
         // Q divides r and j < Q: input m lives in CTA (m*Q)/r at local offset
         // B*j + B*((m*Q) % r) + tl + TL*u -- compile-time owners and offsets.
-        const int lbase = padpos(B * j + tl);
+        const int lbase = padpos<PS>(B * j + tl);
 #pragma unroll
         for (int m = 0; m < r; m++) {
             const int owner = (m * Q) / r;
             const int lq = (m * Q) % r;
-            const float2 *b = cg::this_cluster().map_shared_rank(region, owner) + lbase + B * lq + B * lq / 16;
+            const float2 *b = cg::this_cluster().map_shared_rank(region, owner) + lbase + B * lq + B * lq / PN;
 #pragma unroll
             for (int u = 0; u < NB; u++)
-                v[u * r + m] = b[TL * u + TL * u / 16];
+                v[u * r + m] = b[TL * u + TL * u / PN];
         }
     } else {
 #pragma unroll
@@ -419,7 +435,7 @@ __device__ __forceinline__ void stage_read(float2 *region, float2 (&v)[R], int j
             const float2 *b = Q > 1 ? cg::this_cluster().map_shared_rank(region, owner) : region;
 #pragma unroll
             for (int u = 0; u < NB; u++)
-                v[u * r + m] = b[padpos(B * lq + tl + TL * u)];
+                v[u * r + m] = b[padpos<PS>(B * lq + tl + TL * u)];
         }
     }
 }
@@ -442,8 +458,9 @@ template <int V> struct Int {
 // Start of a kernel launched by launch_dependent (launch.h): waits until the
 // stream's previous kernel has finished and its writes are visible.  Every CTA
 // of such a kernel passes here before it touches memory that another kernel
-// writes, and reads such memory by ordinary loads (ld_data, ld_policy), never
-// by the read-only path, which a compiler may move across the wait.
+// writes, and reads such memory by ordinary loads (ld_data, ld_policy, or
+// through pointers that are neither const __restrict__ nor __ldg's), never by
+// the read-only path, which a compiler may move across the wait.
 // No kernel triggers its dependents early: their CTAs then come in as its own
 // leave.  With the trigger at the start, before the stores or after the first
 // stage the waiting CTAs crowd the SMs that empty first (c2c 2^19: 15.7, 9.5
@@ -455,16 +472,6 @@ __device__ __forceinline__ float2 ld_data(const float2 *p)
 {
     float2 v;
     asm volatile("ld.global.v2.f32 {%0, %1}, [%2];" : "=f"(v.x), "=f"(v.y) : "l"(p) : "memory");
-    return v;
-}
-
-__device__ __forceinline__ float4 ld_data4(const float4 *p)
-{
-    float4 v;
-    asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];"
-                 : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                 : "l"(p)
-                 : "memory");
     return v;
 }
 
@@ -663,7 +670,8 @@ __device__ __forceinline__ void load_stage0_c2r_rows(const TileArgs &a, const fl
     using S = Sched<L, R>;
     using TT = Tile<L, R, 1>;
     constexpr int r = S::radix(0), NB = R / r, B = TT::B(0), TL = TT::TL;
-    constexpr bool CONST_PAD = B % 16 == 0 && (NB == 1 || TL % 16 == 0);
+    constexpr int PS = S::PS, PN = S::PN;
+    constexpr bool CONST_PAD = B % PN == 0 && (NB == 1 || TL % PN == 0);
     auto off = [](int u, int m) { return TL * u + B * m; };
     const bool valid = tr < a.ntrans;
     const bool mul = a.prologue == PRO_MUL_C2R;
@@ -690,10 +698,10 @@ __device__ __forceinline__ void load_stage0_c2r_rows(const TileArgs &a, const fl
             if (tl == 0)
                 xm = times(xm, gload<COH>(g + L));
         }
-        const int base = padpos(tl);
+        const int base = padpos<PS>(tl);
 #pragma unroll
         for (int q = 0; q < R; q++)
-            region[CONST_PAD ? base + off(q / r, q % r) / 16 * 17 : padpos(tl + off(q / r, q % r))] = v[q];
+            region[CONST_PAD ? base + off(q / r, q % r) / PN * (PN + 1) : padpos<PS>(tl + off(q / r, q % r))] = v[q];
     } else {
 #pragma unroll
         for (int q = 0; q < R; q++)
@@ -702,9 +710,9 @@ __device__ __forceinline__ void load_stage0_c2r_rows(const TileArgs &a, const fl
     __syncthreads();
     if (valid) {
         // the mirror of position tl + o is L - tl - o: a base less a constant
-        // where the offsets o are multiples of the padding's 16
+        // where the offsets o are multiples of the padding's period
         const float2 *w = a.rtw + tl;
-        const int mp = padpos(L - tl);
+        const int mp = padpos<PS>(L - tl);
 #pragma unroll
         for (int q = 0; q < R; q++) {
             const int o = off(q / r, q % r);
@@ -712,7 +720,7 @@ __device__ __forceinline__ void load_stage0_c2r_rows(const TileArgs &a, const fl
             if (q == 0 && tl == 0)
                 xb = xm;  // its mirror X[M] is not staged
             else
-                xb = region[CONST_PAD ? mp - o / 16 * 17 : padpos(L - tl - o)];
+                xb = region[CONST_PAD ? mp - o / PN * (PN + 1) : padpos<PS>(L - tl - o)];
             v[q] = c2r_fixup(v[q], xb, __ldg(w + o));
         }
     }
@@ -784,7 +792,7 @@ template <int L, int R, int C, int Q, int LMAP, int SMAP>
 __host__ __device__ constexpr size_t tile_exchange_bytes()
 {
     return (Sched<L, R>::NST > 1)
-               ? (size_t)C * region_stride<L / Q, C, (LMAP == ACROSS || SMAP == ACROSS)>() * sizeof(float2)
+               ? (size_t)C * region_stride<L / Q, C, (LMAP == ACROSS || SMAP == ACROSS), Sched<L, R>::PS>() * sizeof(float2)
                : 0;
 }
 
@@ -827,7 +835,7 @@ __device__ __forceinline__ void run_stages(float2 (&v)[R], int j, int &c, int &t
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
     if constexpr (s < S::NST) {
-        constexpr int RS = region_stride<TT::LQ, C, (LMAP == ACROSS || SMAP == ACROSS)>();
+        constexpr int RS = region_stride<TT::LQ, C, (LMAP == ACROSS || SMAP == ACROSS), S::PS>();
         stage_write<L, R, Q, s - 1>(smem + c * RS, v, j, tl);
         tile_sync<Q>();
         split_tid<(s == S::NST - 1) ? SMAP : ALONG, C, TT::TL>(threadIdx.x, c, tl);
@@ -869,7 +877,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
     using S = Sched<L, R>;
     using TT = Tile<L, R, Q>;
     constexpr int TL = TT::TL, NST = S::NST;
-    constexpr int RS = region_stride<TT::LQ, C, (LMAP == ACROSS || SMAP == ACROSS)>();
+    constexpr int RS = region_stride<TT::LQ, C, (LMAP == ACROSS || SMAP == ACROSS), S::PS>();
     static_assert(NST > 1 || LMAP == SMAP, "single-stage tiles cannot change the thread map");
     static_assert(NST > 1 || Q == 1, "single-stage tiles are not split over a cluster");
 
@@ -983,7 +991,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                     const int pos = p0 + TL * u + m * Q * BL;
                     const int owner = pos / LQ;
                     float2 *dst = Q > 1 ? cg::this_cluster().map_shared_rank(region, owner) : region;
-                    dst[padpos(pos - owner * LQ)] = v[u * rl + m];
+                    dst[padpos<S::PS>(pos - owner * LQ)] = v[u * rl + m];
                 }
             tile_sync<Q>();
             if (Q == 1 && valid) {
@@ -992,19 +1000,20 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                 // X[M+k] = hi, X[2M-k] = conj(lo) for the full output), so a
                 // thread resolves k < M/2 and reads each value once.
                 // Positions k and M - k are a base plus and less a constant
-                // where TL is a multiple of the padding's 16.
-                constexpr bool CP = TL % 16 == 0;
-                const int kp = padpos(tl), mp = padpos(M - tl);
+                // where TL is a multiple of the padding's period.
+                constexpr int PS = S::PS, PN = S::PN;
+                constexpr bool CP = TL % PN == 0;
+                const int kp = padpos<PS>(tl), mp = padpos<PS>(M - tl);
                 float2 *olo = out + obase + (long long)tl * os, *ohi = out + obase + (long long)(M - tl) * os;
                 const float2 *rt = a.rtw + tl;
 #pragma unroll
                 for (int q = 0; q < R / 2; q++) {
                     const int k = tl + TL * q;
-                    const float2 zk = region[CP ? kp + TL * q / 16 * 17 : padpos(k)];
+                    const float2 zk = region[CP ? kp + TL * q / PN * (PN + 1) : padpos<PS>(k)];
                     if (k == 0) {
                         out[obase] = make_float2(zk.x + zk.y, 0.f);
                         out[obase + (long long)M * os] = make_float2(zk.x - zk.y, 0.f);
-                        const float2 zh = region[padpos(M / 2)];  // the middle bin pairs with itself
+                        const float2 zh = region[padpos<PS>(M / 2)];  // the middle bin pairs with itself
                         float2 lo, hi;
                         r2c_bins(zh, zh, __ldg(&a.rtw[M / 2]), lo, hi);
                         out[obase + (long long)(M / 2) * os] = lo;
@@ -1012,7 +1021,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                             out[obase + (long long)(M / 2 + M) * os] = hi;
                     } else {
                         float2 lo, hi;
-                        const float2 zm = region[CP ? mp - TL * q / 16 * 17 : padpos(M - k)];
+                        const float2 zm = region[CP ? mp - TL * q / PN * (PN + 1) : padpos<PS>(M - k)];
                         r2c_bins(zk, zm, __ldg(rt + TL * q), lo, hi);
                         olo[(long long)(TL * q) * os] = lo;
                         ohi[-(long long)(TL * q) * os] = cconj(hi);
@@ -1027,7 +1036,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                 for (int q = 0; q < R; q++) {
                     const int kl = tl + TL * q;  // local position in this CTA's slice
                     const int k = j * LQ + kl;
-                    const float2 zk = region[padpos(kl)];
+                    const float2 zk = region[padpos<S::PS>(kl)];
                     if (k == 0) {
                         out[obase] = make_float2(zk.x + zk.y, 0.f);
                         out[obase + (long long)M * a.out_stride] = make_float2(zk.x - zk.y, 0.f);
@@ -1035,7 +1044,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                         const int mk = M - k, mo = mk / LQ;
                         const float2 *src = Q > 1 ? cg::this_cluster().map_shared_rank(region, mo) : region;
                         float2 lo, hi;
-                        r2c_bins(zk, src[padpos(mk - mo * LQ)], __ldg(&a.rtw[k]), lo, hi);
+                        r2c_bins(zk, src[padpos<S::PS>(mk - mo * LQ)], __ldg(&a.rtw[k]), lo, hi);
                         out[obase + (long long)k * a.out_stride] = lo;
                         if (full)
                             out[obase + (long long)(k + M) * a.out_stride] = hi;

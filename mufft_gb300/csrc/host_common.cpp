@@ -299,9 +299,9 @@ bool device_prepare(int *dev_out)
             }
         for (int p : kStage32Sizes)
             for (int k = 0; k < p; k++)
-                for (int e = 0; e < 5; e++) {
+                for (int e = 0; e < 8; e++) {
                     const long long n = 32ll * p;
-                    double ph = -2.0 * M_PI * (double)(((long long)(1 << e) * k) % n) / (double)n;
+                    double ph = -2.0 * M_PI * (double)(((long long)kStage32Exps[e] * k) % n) / (double)n;
                     h[stage32_base(p) + 8 * k + e] = make_float2((float)std::cos(ph), (float)std::sin(ph));
                 }
         if (!cuda_ok(cudaMalloc(&ds.tw, h.size() * sizeof(float2)), "cudaMalloc(twiddles)"))

@@ -79,11 +79,11 @@ __global__ void __launch_bounds__(256) adjoint_filter_reduce(float2 *acc, float2
         const float2 *gi = g + (long long)i0 * gdist, *ai = a + (long long)i0 * adist;
 #pragma unroll 4
         for (unsigned i = i0; i < i1; i++) {
-            const float2 gk = ld_data(gi + k), ak = ld_data(ai + k);
+            const float2 gk = gi[k], ak = ai[k];
             sum.x += gk.x * ak.x + gk.y * ak.y;  // G conj(A)
             sum.y += gk.y * ak.x - gk.x * ak.y;
             if (stereo) {
-                const float2 gm = ld_data(gi + km), am = ld_data(ai + km);
+                const float2 gm = gi[km], am = ai[km];
                 sum.x += gm.x * am.x + gm.y * am.y;  // conj(G conj(A)) at N-k
                 sum.y -= gm.y * am.x - gm.x * am.y;
             }
@@ -113,7 +113,7 @@ __global__ void __launch_bounds__(256) adjoint_filter_sum(float2 *acc, const flo
         float2 sum = make_float2(0.f, 0.f);
 #pragma unroll 8
         for (unsigned y = 0; y < rows; y++)
-            sum = cadd(sum, ld_data(part + (size_t)y * nb + k));
+            sum = cadd(sum, part[(size_t)y * nb + k]);
         float2 r = cscale(sum, f);
         if (accumulate)
             r = cadd(r, acc[k]);

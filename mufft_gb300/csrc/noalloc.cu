@@ -45,7 +45,7 @@ static __device__ __align__(256) float2 g_noalloc_scratch[kNoAllocMaxPoints];
 static __device__ __align__(256) float2 g_noalloc_twiddles[kStageTableFloat2];
 
 // Stage twiddle table (layout: common.h, stage_table_base) in FP64, rounded
-// once to float: entry (r, p, k, e) = exp(-2*pi*i * (2^e * k mod r*p) / (r*p)).
+// once to float: entry (r, p, k, e) = exp(-2*pi*i * (e * k mod r*p) / (r*p)).
 __global__ void noalloc_fill_twiddles(float2 *t)
 {
     const int n = kStageTableFloat2;
@@ -55,18 +55,19 @@ __global__ void noalloc_fill_twiddles(float2 *t)
             const int per_radix = kStageTableK * 4;
             const int ri = idx / per_radix;
             const int kk = (idx % per_radix) / 4;
-            e = idx % 4;
+            e = 1 << (idx % 4);
             r = 2 << ri;
             p = kk < 16 ? 16 : (kk < 272 ? 256 : 4096);
             k = kk - stage_p_offset(p);
         } else {
-            e = (idx - kStage32Begin) % 8;
+            constexpr int exps[8] = {1, 2, 4, 8, 3, 12, 16, 0};  // kStage32Exps
+            e = exps[(idx - kStage32Begin) % 8];
             r = 32;
-            p = idx < stage32_base(256) ? 16 : idx < stage32_base(512) ? 256 : 512;
+            p = idx < stage32_base(32) ? 16 : idx < stage32_base(256) ? 32 : idx < stage32_base(512) ? 256 : 512;
             k = (idx - stage32_base(p)) / 8;
         }
         const long long rp = (long long)r * p;
-        const long long m = ((long long)(1 << e) * k) % rp;
+        const long long m = ((long long)e * k) % rp;
         double s, c;
         sincospi(2.0 * (double)m / (double)rp, &s, &c);
         t[idx] = make_float2((float)c, (float)-s);

@@ -63,8 +63,10 @@ mufft_plan_2d *create_2d(int kind, unsigned Nx, unsigned Ny, int direction, unsi
         set_error(MUFFT_GB_ERR_UNSUPPORTED, "2D side longer than %u", kMaxSinglePass);
         return nullptr;
     }
-    const TileKernel *krow = find_tile((int)Mx, ALONG, ALONG);
-    const TileKernel *kcol = find_tile((int)Ny, ACROSS, ACROSS);
+    const TileKernel *krow = choose_tile((int)Mx, ALONG, ALONG, Ny, 1);
+    // columns the column pass transforms
+    const unsigned ncol = kind == K2_C2C || (kind == K2_R2C && (flags & MUFFT_FLAG_FULL_R2C)) ? Nx : Mx + 1;
+    const TileKernel *kcol = choose_tile((int)Ny, ACROSS, ACROSS, ncol, 1);
     if (!krow || !kcol) {
         set_error(MUFFT_GB_ERR_UNSUPPORTED, "no 2D kernels for %u x %u", Nx, Ny);
         return nullptr;
@@ -187,12 +189,17 @@ mufft_plan_2d *create_2d(int kind, unsigned Nx, unsigned Ny, int direction, unsi
     // 41.1 / 44.7 / 63.0 and 4096 x 2048 or 16384 x 2048 slower in every
     // kind.  So the automatic choice: Ny >= 8192, or Ny = 4096 with Nx >= 4096
     // (real) / Nx >= 8192 (c2c); without the hints one pass up to 4096.
+    // And Ny = 4096 with fewer than 400 columns, where one pass would have
+    // fewer than 100 CTAs: 128 x 4096 13.3 / 14.1 / 13.3 -> 8.2 / 8.4 / 8.2,
+    // 512 x 4096 r2c / c2r 15.7 / 17.3 -> 14.3 / 15.4 (c2c, 128 CTAs, would lose:
+    // 17.4 -> 18.3).
     const int mode = opt_cols2d();
     const unsigned lgy = ilog2u(Ny);
     const unsigned N1 = 1u << (lgy / 2), N2 = Ny / N1;
     const TileKernel *kc1 = find_tile((int)N1, ACROSS, ACROSS), *kc2 = find_tile((int)N2, ACROSS, ACROSS);
     const bool wide = opt_l2() == 1 && Ny >= 4096 && Nx >= (kind == K2_C2C ? 8192u : 4096u);
-    if ((mode == 2 || (mode == 0 && (Ny >= 8192 || wide))) && N1 >= 2 && kc1 && kc2) {
+    const bool few = Ny == 4096 && ncol < 400;
+    if ((mode == 2 || (mode == 0 && (Ny >= 8192 || wide || few))) && N1 >= 2 && kc1 && kc2) {
         const unsigned ncols = (unsigned)col.a.ntrans;
         const long long s_in = col.a.in_stride;                                 // pitch the columns are read at
         const long long s_out = kind == K2_C2R ? col.a.out_stride : (long long)Nx;  // pitch of C1 / C2 outputs

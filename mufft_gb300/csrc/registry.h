@@ -41,4 +41,11 @@ void register_tiles_transpose(std::vector<TileKernel> &out);
 // first registered.  nullptr if none exists.
 const TileKernel *find_tile(int L, int lmap, int smap, int C = 0, int R = 0, int Q = 0);
 
+// The instantiation for a pass of `rows` grid rows of `ntrans` transforms:
+// find_tile's where the plan's options prefer one (or ask for a form that
+// only some tiles have), else the measured choice for the pass's size.
+// real: a row pass with an r2c or c2r fix-up.
+const TileKernel *choose_tile(int L, int lmap, int smap, unsigned long long ntrans, unsigned long long rows,
+                              bool real = false);
+
 }  // namespace mgb

@@ -20,6 +20,79 @@
 
 namespace mgb {
 
+// Measured tile choices (us, GB300): a pass whose default tile (the first
+// registered) would launch at least `from` and fewer than `below` CTAs takes
+// C transforms per tile and R elements per thread instead.
+namespace {
+
+constexpr unsigned kAny = ~0u;
+// two CTAs per SM: below, a narrower tile spreads the pass over more SMs
+constexpr unsigned kFill = 2 * 152;
+
+struct TileRule {
+    int L, lmap, smap, C, R;
+    unsigned from, below;
+};
+
+const TileRule kTileRules[] = {
+    // Rows: one or two warps per tile.  Their barriers hold back fewer threads,
+    // and the SMs are filled more evenly: 2^24 points as rows of 512 c2c / r2c /
+    // c2r 44.9 / 53.2 / 56.5 -> 40.1 / 44.1 / 47.9 (also one exchange fewer, 16 x
+    // 32), of 256 41.2 / 44.9 / 46.9 -> 40.5 / 41.3 / 43.3, of 128 40.8 / 48.5 /
+    // 50.7 -> 40.0 / 46.4 / 48.4, of 64 46.5 / 59.6 / 59.9 -> 45.3 / 57.4 / 58.1;
+    // 2^18 points as rows of 16 .. 512 2.7-5.7 -> 2.6-3.3
+    {512, ALONG, ALONG, 2, 32, 0, kAny},
+    {256, ALONG, ALONG, 4, 16, 0, kAny},
+    {128, ALONG, ALONG, 8, 16, 0, kAny},
+    {64, ALONG, ALONG, 16, 16, 0, kAny},
+    {32, ALONG, ALONG, 64, 16, 0, kAny},
+    {16, ALONG, ALONG, 64, 16, 0, kAny},
+    // Columns: 32 elements a thread save an exchange at 512 (16 x 32) and 1024
+    // points (32 x 32).  c2c 2^20 x 32 203 -> 192, with the rows below 181;
+    // 2^18 x 64 94.0 -> 81.1 and 2^19 x 64 189 -> 162 with 16 columns, which
+    // need enough of them (2^19 x 3: 14.2 against 13.4 with 8)
+    {512, ACROSS, ACROSS, 16, 32, 2 * kFill, kAny},
+    {512, ACROSS, ACROSS, 8, 32, 0, 2 * kFill},
+    {1024, ACROSS, ACROSS, 8, 32, 0, kAny},
+    {256, ACROSS, ACROSS, 8, 16, 0, kFill},  // 2^16 x 1: 5.3 -> 4.8
+    {128, ACROSS, ACROSS, 16, 16, 0, kAny},  // 2^22 x 1: 31.4 -> 29.8, x 8 234.7 -> 233.6
+    // and as the columns of a grid: c2r 1024 x 64 5.3 -> 5.0, r2c 1024 x 128
+    // 5.0 -> 4.4, c2c 2048 x 2048 30.6 -> 28.5 (but r2c 1024 x 2048, 129 tiles
+    // of four, 11.2 -> 13.4)
+    {64, ACROSS, ACROSS, 32, 16, 0, kAny},
+    {2048, ACROSS, ACROSS, 8, 16, 256, kAny},
+    // Rows stored transposed: 2^17 x 61 40.0 -> 36.3, 2^21 x 16 200.1 -> 196.0
+    {256, ALONG, ACROSS, 8, 16, 0, kFill},
+    {512, ALONG, ACROSS, 8, 32, 0, kAny},
+    {1024, ALONG, ACROSS, 8, 32, 0, kAny},
+    {2048, ALONG, ACROSS, 4, 32, 0, kAny},
+};
+
+}  // namespace
+
+const TileKernel *choose_tile(int L, int lmap, int smap, unsigned long long ntrans, unsigned long long rows, bool real)
+{
+    const TileKernel *k = find_tile(L, lmap, smap);
+    if (!k || opt_tma() || opt_stream() == 1)
+        return k;
+    if (t_opts)
+        for (const TileKernel &t : t_opts->tiles)
+            if (t.L == L && t.lmap == lmap && t.smap == smap)
+                return k;
+    const unsigned long long ctas = (ntrans + k->C - 1) / k->C * rows;
+    for (const TileRule &r : kTileRules)
+        if (r.L == L && r.lmap == lmap && r.smap == smap && ctas >= r.from && (r.below == kAny || ctas < r.below))
+            if (const TileKernel *t = find_tile(L, lmap, smap, r.C, r.R, 1))
+                return t;
+    // real rows of 1024 as 32 x 32 where there are enough of them (2048-real
+    // frames x 4096 r2c / c2r 15.4 / 16.9 -> 14.3 / 16.0, x 16384 47.1 -> 43.1,
+    // but x 300 2.6 -> 2.8)
+    if (real && L == 1024 && lmap == ALONG && smap == ALONG && ctas >= 1024)
+        if (const TileKernel *t = find_tile(L, lmap, smap, 1, 32, 1))
+            return t;
+    return k;
+}
+
 static const void *pick(Role r, const Buffers &b)
 {
     switch (r) {
@@ -473,7 +546,8 @@ bool build_fft_passes(const FftSpec &s, const float2 *tw, PlanResources &res, bo
     const unsigned M = s.M;
     const bool r2c = s.epilogue == EPI_R2C || s.epilogue == EPI_R2C_FULL;
     if (M <= kMaxSinglePass) {
-        const TileKernel *k = find_tile((int)M, ALONG, ALONG);
+        const bool real = r2c || s.prologue == PRO_C2R || s.prologue == PRO_MUL_C2R;
+        const TileKernel *k = choose_tile((int)M, ALONG, ALONG, s.batch, 1, real);
         if (!k) {
             set_error(MUFFT_GB_ERR_UNSUPPORTED, "no tile kernel for length %u", M);
             return false;
@@ -622,9 +696,9 @@ bool build_fft_passes(const FftSpec &s, const float2 *tw, PlanResources &res, bo
             set_error(MUFFT_GB_ERR_UNSUPPORTED, "batch %u too large for three-level lengths", s.batch);
             return false;
         }
-        const TileKernel *ka = find_tile((int)N1, ACROSS, ACROSS);
-        const TileKernel *kb = find_tile((int)N2, ACROSS, ACROSS);
-        const TileKernel *kr = find_tile((int)N3, ALONG, ACROSS);
+        const TileKernel *ka = choose_tile((int)N1, ACROSS, ACROSS, MR, s.batch);
+        const TileKernel *kb = choose_tile((int)N2, ACROSS, ACROSS, N3, (unsigned long long)N1 * s.batch);
+        const TileKernel *kr = choose_tile((int)N3, ALONG, ACROSS, N1, (unsigned long long)N2 * s.batch);
         if (!ka || !kb || !kr) {
             set_error(MUFFT_GB_ERR_UNSUPPORTED, "no three-level kernels for %u x %u x %u", N1, N2, N3);
             return false;
@@ -721,8 +795,8 @@ bool build_fft_passes(const FftSpec &s, const float2 *tw, PlanResources &res, bo
         set_error(MUFFT_GB_ERR_UNSUPPORTED, "batch %u too large for multi-pass lengths", s.batch);
         return false;
     }
-    const TileKernel *kc = find_tile((int)N1, ACROSS, ACROSS);
-    const TileKernel *kr = find_tile((int)N2, ALONG, ACROSS);
+    const TileKernel *kc = choose_tile((int)N1, ACROSS, ACROSS, N2, s.batch);
+    const TileKernel *kr = choose_tile((int)N2, ALONG, ACROSS, N1, s.batch);
     if (!kc || !kr) {
         set_error(MUFFT_GB_ERR_UNSUPPORTED, "no four-step kernels for %u x %u", N1, N2);
         return false;

@@ -35,6 +35,14 @@ void register_tiles_across(std::vector<TileKernel> &out)
     TILE(4096, 32, 2);
     TILE(8192, 32, 2);
     TILE(16384, 32, 1);
+    // further shapes, chosen by size (choose_tile)
+    TILE(64, 16, 32);
+    TILE(128, 16, 16);
+    TILE(256, 16, 8);
+    TILE(512, 32, 16);
+    TILE(512, 32, 8);
+    TILE(1024, 32, 8);
+    TILE(2048, 32, 4);
 }
 
 }  // namespace mgb

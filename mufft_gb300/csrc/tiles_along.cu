@@ -32,9 +32,7 @@ void register_tiles_along(std::vector<TileKernel> &out)
     // 32 elements a thread and radix-32 stages: one exchange fewer than with 16
     // (c2c 2048 x 8192: 62.9 -> 48.3 us, c2r 3001 x 16384 reals 109.9 -> 92.8,
     // r2c 2048 x 16384 reals 70.5 -> 62.8, c2c 1024 x 16384: 78.6 -> 71.2; one
-    // transform alone the same).  512 points gain for c2c (16384 x 512: 24.8 ->
-    // 23.3) but not for real data (29.0 -> 29.5), and as 32 x 32 1024 points
-    // lose (4096 x 1024: 12.8 -> 15.7 us).
+    // transform alone the same)
     TILE(8192, 32, 1);
     TILE(8192, 16, 1);
     TILE_Q(8192, 16, 1, 2);  // clusters: the transform is spread over Q SMs
@@ -43,12 +41,18 @@ void register_tiles_along(std::vector<TileKernel> &out)
     TILE_Q(16384, 16, 1, 4);
     TILE_Q(32768, 16, 1, 8);
     TILE_Q(65536, 16, 1, 8);
-    // wider batched tiles (after the defaults above), for the autotuner and
+    // further shapes, for the choices by size (choose_tile), the autotuner and
     // explicit tile choices
+    TILE(16, 16, 64);
+    TILE(32, 16, 64);
+    TILE(64, 16, 16);
+    TILE(128, 16, 8);
+    TILE(256, 16, 4);
+    TILE(512, 32, 2);
+    TILE(1024, 32, 1);
     TILE(1024, 16, 4);
     TILE(1024, 16, 2);
     TILE(2048, 16, 2);
-    TILE(512, 32, 16);
 }
 
 }  // namespace mgb

@@ -31,6 +31,11 @@ void register_tiles_transpose(std::vector<TileKernel> &out)
     TILE(4096, 32, 2);
     TILE(8192, 32, 2);
     TILE(16384, 32, 1);
+    // further shapes, chosen by size (choose_tile)
+    TILE(256, 16, 8);
+    TILE(512, 32, 8);
+    TILE(1024, 32, 8);
+    TILE(2048, 32, 4);
 }
 
 }  // namespace mgb

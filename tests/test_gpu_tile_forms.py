@@ -74,7 +74,7 @@ def test_column_twiddle_forms(gpu, torch, mode):
     assert rel_l2(got, ref) <= 2.0 ** -23 * 17
 
 
-@pytest.mark.parametrize("tile", [(512, 0, 0, 16, 32, 1), (512, 0, 0, 8, 16, 1), (8192, 0, 0, 1, 32, 1),
+@pytest.mark.parametrize("tile", [(512, 0, 0, 2, 32, 1), (512, 0, 0, 8, 16, 1), (1024, 0, 0, 1, 32, 1), (8192, 0, 0, 1, 32, 1),
                                   (8192, 0, 0, 1, 16, 1), (16384, 0, 0, 1, 32, 1), (16384, 0, 0, 1, 16, 1)])
 @pytest.mark.parametrize("kind", [0, 1, 2])
 def test_wide_radix_rows(gpu, torch, tile, kind):
