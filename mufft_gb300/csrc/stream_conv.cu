@@ -29,6 +29,7 @@ namespace mgb {
 namespace {
 
 constexpr int kWarps = 8;
+constexpr int kBatch = 8;  // partitions a warp has in flight
 constexpr unsigned kBins = 64;  // per group: two per lane
 
 __device__ __forceinline__ void cmac2(float4 &acc, const float4 a, const float4 b)
@@ -101,7 +102,12 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
     const unsigned lane = threadIdx.x & 31, w = threadIdx.x >> 5;
 
     if (blockIdx.x == 0) {
-        tile_body<M, 16, C, 1, ALONG, ALONG, false>(a.fwd, 0, 0, 0, 0, smem);
+        if (a.inv_c2r_rows)
+            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, false, FL_R2C>(a.fwd, 0, 0, 0, 0,
+                                                                                                  smem);
+        else
+            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, false, FL_PLAIN>(a.fwd, 0, 0, 0, 0,
+                                                                                                    smem);
         __syncthreads();  // the spectrum is written and the whole window has been read
         if (threadIdx.x == 0)
             st_release(&a.tickets[2], k + 1);
@@ -118,11 +124,22 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
     const unsigned p1 = 1 + (unsigned)((unsigned long long)np * (g + 1) / a.G);
     const unsigned b = x * kBins + 2 * lane;
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
-#pragma unroll 8
-    for (unsigned p = p0 + w; p < p1; p += kWarps) {
-        const unsigned slot = cur >= p ? cur - p : cur + a.P - p;  // block k - p
-        cmac2(acc, ld_data4((const float4 *)&a.fdl[(size_t)slot * a.pitch + b]),
-              __ldg((const float4 *)&a.h[(size_t)p * a.pitch + b]));
+    // kBatch partitions' loads in flight at once, the last batch short
+    for (unsigned pb = p0 + w; pb < p1; pb += kWarps * kBatch) {
+        float4 xv[kBatch], hv[kBatch];
+#pragma unroll
+        for (int i = 0; i < kBatch; i++) {
+            const unsigned p = pb + kWarps * i;
+            if (p < p1) {
+                const unsigned slot = cur >= p ? cur - p : cur + a.P - p;  // block k - p
+                xv[i] = *(const float4 *)&a.fdl[(size_t)slot * a.pitch + b];
+                hv[i] = __ldg((const float4 *)&a.h[(size_t)p * a.pitch + b]);
+            }
+        }
+#pragma unroll
+        for (int i = 0; i < kBatch; i++)
+            if (pb + kWarps * i < p1)
+                cmac2(acc, xv[i], hv[i]);
     }
     red[w][lane] = acc;
     __syncthreads();
@@ -185,7 +202,8 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
         if (a.inv_c2r_rows)
             tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, true, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0, smem);
         else
-            tile_body<M, 16, C, 1, ALONG, ALONG, true>(a.inv, 0, 0, 0, 0, smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, false, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0,
+                                                                                                   smem);
         if (threadIdx.x == 0) {
             a.tickets[1] = 0;  // read again by the next launch only
             a.tickets[0] = k + 1;

@@ -58,6 +58,23 @@ void destroy_stream_conv(mufft_gb_stream_conv *c)
     delete c;
 }
 
+// Partition ranges per bin group of a one-launch block.  A range CTA's eight
+// warps take eight partitions each at a time: 64 partitions are one batch of
+// loads, and more ranges only add partial sums for the group's last CTA to
+// read back (us per block, as many ranges as fit / this rule: stereo 1024 x
+// 2^20 taps 8.7 / 8.5, x 369562 taps 7.9 / 7.4, x 100000 7.6 / 6.6, stereo 256 x
+// 2^18 7.5 / 6.9, mono 512 x 2^20 8.4 / 8.1).  128 where ranges of 64 do not
+// fit.  With few groups the sums are short, and smaller ranges pay (stereo 128
+// x 40000 7.2 / 6.2, mono 64 x 5000 7.7 / 6.2).
+unsigned auto_ranges(unsigned P, unsigned groups, unsigned max_g)
+{
+    const unsigned np = P > 1 ? P - 1 : 1;
+    if (groups <= 4)
+        return std::max((np + 31) / 32, std::min(8u, (np + 7) / 8));
+    const unsigned g = (np + 63) / 64;
+    return g <= max_g ? g : (np + 127) / 128;
+}
+
 }  // namespace
 
 extern "C" {
@@ -140,7 +157,8 @@ mufft_gb_stream_conv *mufft_gb_create_stream_conv(unsigned block, unsigned metho
         // it finishes the group); all CTAs resident at once
         const unsigned slots = (unsigned)std::max(2, sms * std::max(per_sm, 1));
         const unsigned max_g = std::max(1u, (slots - 1) / upols_groups(nb));
-        c->G = std::max(1u, std::min({want_ranges ? want_ranges : max_g, max_g, std::max(P - 1, 1u)}));
+        c->G = std::max(1u, std::min({want_ranges ? want_ranges : auto_ranges(P, upols_groups(nb), max_g), max_g,
+                                      std::max(P - 1, 1u)}));
     } else {
         c->G = want_ranges ? std::min(want_ranges, P) : upols_chunks(nb, P, sms);
     }
