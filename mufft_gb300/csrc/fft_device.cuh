@@ -524,32 +524,45 @@ __device__ __forceinline__ void st_policy(float2 *p, float2 v, unsigned long lon
 // decides both at run time, with every form compiled in; the others fix them,
 // so that a launch pays no per-element tests and holds less code.  All of
 // them read whole plain inputs (PRO_PLAIN, no `half`).
+// A form is a prologue, whether the input is zero-padded, an epilogue and the
+// four-step twiddle it applies (1: column powers, 2: by grid row).
+__host__ __device__ constexpr int form(int prologue, int half, int epilogue, int twiddle = 0)
+{
+    return 1 | prologue << 1 | half << 3 | epilogue << 4 | twiddle << 6;
+}
 enum Flavour : int {
     FL_ANY = 0,
-    FL_PLAIN = 1,   // EPI_PLAIN
-    FL_COLPOW = 2,  // EPI_TWIDDLE with tw_colpow
-    FL_BYROW = 3,   // EPI_TWIDDLE with tw_by_y
-    FL_R2C = 4,     // EPI_R2C
+    FL_PLAIN = form(PRO_PLAIN, 0, EPI_PLAIN),
+    FL_COLPOW = form(PRO_PLAIN, 0, EPI_TWIDDLE, 1),
+    FL_BYROW = form(PRO_PLAIN, 0, EPI_TWIDDLE, 2),
+    FL_R2C = form(PRO_PLAIN, 0, EPI_R2C),
+    FL_HALF_PLAIN = form(PRO_PLAIN, 1, EPI_PLAIN),
+    FL_HALF_R2C = form(PRO_PLAIN, 1, EPI_R2C),
+    FL_HALF_COLPOW = form(PRO_PLAIN, 1, EPI_TWIDDLE, 1),
+    FL_MUL_PLAIN = form(PRO_MUL, 0, EPI_PLAIN),
+    FL_MUL_COLPOW = form(PRO_MUL, 0, EPI_TWIDDLE, 1),
+    FL_C2R_COLPOW = form(PRO_C2R, 0, EPI_TWIDDLE, 1),
+    FL_MUL_C2R_COLPOW = form(PRO_MUL_C2R, 0, EPI_TWIDDLE, 1),
 };
 template <int FL> __device__ __forceinline__ int fl_prologue(const TileArgs &a)
 {
-    return FL == FL_ANY ? a.prologue : (int)PRO_PLAIN;
+    return FL == FL_ANY ? a.prologue : (FL >> 1 & 3);
 }
-template <int FL> __device__ __forceinline__ int fl_half(const TileArgs &a) { return FL == FL_ANY ? a.half : 0; }
+template <int FL> __device__ __forceinline__ int fl_half(const TileArgs &a)
+{
+    return FL == FL_ANY ? a.half : (FL >> 3 & 1);
+}
 template <int FL> __device__ __forceinline__ int fl_epilogue(const TileArgs &a)
 {
-    return FL == FL_ANY      ? a.epilogue
-           : FL == FL_PLAIN  ? (int)EPI_PLAIN
-           : FL == FL_R2C    ? (int)EPI_R2C
-                             : (int)EPI_TWIDDLE;
+    return FL == FL_ANY ? a.epilogue : (FL >> 4 & 3);
 }
 template <int FL> __device__ __forceinline__ bool fl_byrow(const TileArgs &a)
 {
-    return FL == FL_ANY ? a.tw_by_y != 0 : FL == FL_BYROW;
+    return FL == FL_ANY ? a.tw_by_y != 0 : FL >> 6 == 2;
 }
 template <int FL> __device__ __forceinline__ bool fl_colpow(const TileArgs &a)
 {
-    return FL == FL_ANY ? a.tw_colpow != 0 : FL == FL_COLPOW;
+    return FL == FL_ANY ? a.tw_colpow != 0 : FL >> 6 == 1;
 }
 
 template <int L, int R, int Q, int LMAP, bool COH = false, int FL = FL_ANY>
@@ -563,7 +576,7 @@ __device__ __forceinline__ void load_stage0(const TileArgs &a, const float2 *__r
     const int mlim = fl_half<FL>(a) ? r / 2 : r;  // zero-padded upper half: inputs m >= r/2 stay zero
     // (zeroed up front by the kernels of many forms: a zeroing under the tests
     // made the ragged kernels spill kilobytes)
-    if (FL == FL_ANY || tr >= a.ntrans) {
+    if (FL == FL_ANY || (FL >> 3 & 1) || tr >= a.ntrans) {
 #pragma unroll
         for (int q = 0; q < R; q++)
             v[q] = make_float2(0.f, 0.f);
@@ -606,43 +619,60 @@ __device__ __forceinline__ void load_stage0(const TileArgs &a, const float2 *__r
     }
     case PRO_MUL: {
         const float2 *g = in2 + ((a.in2_bcast & 2) ? 0 : tbase) + p0 * sst;
+        const float cs = a.conj2 ? -1.f : 1.f;
+        const long long mstep = (long long)(Q * B) * sst, ustep = (long long)TL * sst;
 #pragma unroll
-        for (int u = 0; u < NB; u++)
+        for (int u = 0; u < NB; u++) {
+            const float2 *fs = f + u * ustep, *gs = g + u * ustep;
 #pragma unroll
-            for (int m = 0; m < r; m++)
-                if (m < mlim) {
-                    const long long o = (long long)(TL * u + m * Q * B) * sst;
-                    float2 gv = gload<COH>(g + o);
-                    gv.y = a.conj2 ? -gv.y : gv.y;
-                    v[u * r + m] = cscale(cmul(gload<COH>(f + o), gv), a.scale);
+            for (int m = 0; m < r; m++) {
+                if (FL != FL_ANY || m < mlim) {
+                    float2 gv = gload<COH>(gs);
+                    gv.y *= cs;
+                    v[u * r + m] = cscale(cmul(gload<COH>(fs), gv), a.scale);
                 }
+                fs += mstep;
+                gs += mstep;
+            }
+        }
         break;
     }
     default: {
         // c2r fix-ups: X[local] and X[M - local] with local = tr*ldist + pos*stride
         const long long tb = tbase - (long long)tr * a.mirror_ldist;
         const long long lfirst = (long long)tr * a.mirror_ldist + p0 * a.in_stride;
-        const bool mul = a.prologue == PRO_MUL_C2R;
+        const bool mul = fl_prologue<FL>(a) == PRO_MUL_C2R;
+        const long long i2 = (a.in2_bcast & 2) ? tb : 0;  // (single-pass: tb is the transform's base)
+        const long long ib0 = tb + a.mirror_len - lfirst;
+        const long long mstep = (long long)(Q * B) * a.in_stride, ustep = (long long)TL * a.in_stride;
+        const float cs = a.conj2 ? -1.f : 1.f;
 #pragma unroll
-        for (int u = 0; u < NB; u++)
+        for (int u = 0; u < NB; u++) {
+            // X[local] upwards and X[M - local] downwards, the same offsets in the second spectrum
+            const float2 *fa = in + tb + lfirst + u * ustep, *fb = in + ib0 - u * ustep;
+            const float2 *w = a.rtw + lfirst + u * ustep;
+            const float2 *ha = mul ? in2 + (tb + lfirst - i2) + u * ustep : nullptr;
+            const float2 *hb = mul ? in2 + (ib0 - i2) - u * ustep : nullptr;
 #pragma unroll
-            for (int m = 0; m < r; m++)
-                if (m < mlim) {
-                    const long long local = lfirst + (long long)(TL * u + m * Q * B) * a.in_stride;
-                    const long long ia = tb + local, ib = tb + a.mirror_len - local;
-                    float2 xa = gload<COH>(&in[ia]), xb = gload<COH>(&in[ib]);
+            for (int m = 0; m < r; m++) {
+                if (FL != FL_ANY || m < mlim) {
+                    float2 xa = gload<COH>(fa), xb = gload<COH>(fb);
                     if (mul) {
-                        const long long i2 = (a.in2_bcast & 2) ? tb : 0;  // (single-pass: tb is the transform's base)
-                        float2 ga = gload<COH>(&in2[ia - i2]), gb = gload<COH>(&in2[ib - i2]);
-                        if (a.conj2) {
-                            ga.y = -ga.y;
-                            gb.y = -gb.y;
-                        }
+                        float2 ga = gload<COH>(ha), gb = gload<COH>(hb);
+                        ga.y *= cs;
+                        gb.y *= cs;
                         xa = cscale(cmul(xa, ga), a.scale);
                         xb = cscale(cmul(xb, gb), a.scale);
                     }
-                    v[u * r + m] = c2r_fixup(xa, xb, __ldg(&a.rtw[local]));
+                    v[u * r + m] = c2r_fixup(xa, xb, __ldg(w));
                 }
+                fa += mstep;
+                fb -= mstep;
+                ha += mstep;
+                hb -= mstep;
+                w += mstep;
+            }
+        }
         break;
     }
     }
@@ -954,7 +984,7 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
     stage_compute<L, R, Q, 0>(v, j, tl, a.tw);
     // the column powers' base rides in the last stage's twiddles where the
     // kernel has that one epilogue
-    constexpr bool BASE = FL == FL_COLPOW && NST > 1;
+    constexpr bool BASE = FL != FL_ANY && FL >> 6 == 1 && NST > 1;
     run_stages<L, R, C, Q, LMAP, SMAP, 1, BASE>(v, j, c, tl, smem, a.tw, wbase);
     // No CTA of the cluster may leave while others still read its slice.
     if constexpr (Q > 1)
@@ -1244,9 +1274,19 @@ template <int L, int R, int C, int Q, int LMAP, int SMAP> constexpr TileFlavours
         if constexpr (LMAP == ACROSS && SMAP == ACROSS && tile_has_thi<L, R, C, Q, LMAP, SMAP>()) {
             f.colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_COLPOW>;
             f.byrow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_BYROW>;
+            if constexpr (L >= 128 && L <= 2048) {  // first passes of multi-pass transforms
+                f.half_colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_HALF_COLPOW>;
+                f.mul_colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_MUL_COLPOW>;
+                f.c2r_colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_C2R_COLPOW>;
+                f.mul_c2r_colpow = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_MUL_C2R_COLPOW>;
+            }
         }
-        if constexpr (LMAP == ALONG && SMAP == ALONG)
+        if constexpr (LMAP == ALONG && SMAP == ALONG) {
+            f.half_plain = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_HALF_PLAIN>;
+            f.half_r2c = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_HALF_R2C>;
+            f.mul_plain = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_MUL_PLAIN>;
             f.r2c = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_R2C>;
+        }
     }
     return f;
 }

@@ -56,8 +56,11 @@ const std::vector<TileKernel> &tile_table()
 {
     static const std::vector<TileKernel> t = [] {
         std::vector<TileKernel> v;
-        register_tiles_along(v);
-        register_tiles_across(v);
+        register_tiles_along_short(v);
+        register_tiles_along_mid(v);
+        register_tiles_along_long(v);
+        register_tiles_across_short(v);
+        register_tiles_across_long(v);
         register_tiles_transpose(v);
         return v;
     }();

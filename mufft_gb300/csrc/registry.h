@@ -8,12 +8,16 @@
 namespace mgb {
 
 // A tile kernel compiled for one prologue and epilogue (fft_device.cuh,
-// Flavour): plain inputs, and the named epilogue.
+// Flavour), named by them.
 struct TileFlavours {
     const void *plain = nullptr;   // plain stores
     const void *colpow = nullptr;  // four-step twiddle by column powers
     const void *byrow = nullptr;   // four-step twiddle by grid row
     const void *r2c = nullptr;     // r2c fix-up, M + 1 bins
+    // zero-padded inputs
+    const void *half_plain = nullptr, *half_r2c = nullptr, *half_colpow = nullptr;
+    // inputs times a second spectrum, and c2r fix-ups of inputs or such products
+    const void *mul_plain = nullptr, *mul_colpow = nullptr, *c2r_colpow = nullptr, *mul_c2r_colpow = nullptr;
 };
 
 struct TileKernel {
@@ -31,8 +35,11 @@ struct TileKernel {
     const void *fn_c2r = nullptr;  // row tiles: variant staging c2r fix-up rows in shared memory
 };
 
-void register_tiles_along(std::vector<TileKernel> &out);
-void register_tiles_across(std::vector<TileKernel> &out);
+void register_tiles_along_short(std::vector<TileKernel> &out);
+void register_tiles_along_mid(std::vector<TileKernel> &out);
+void register_tiles_along_long(std::vector<TileKernel> &out);
+void register_tiles_across_short(std::vector<TileKernel> &out);
+void register_tiles_across_long(std::vector<TileKernel> &out);
 void register_tiles_transpose(std::vector<TileKernel> &out);
 
 // Returns the instantiation for (L, lmap, smap): the one matching the

@@ -177,17 +177,21 @@ static const void *tile_fn(const Pass &p)
     if (uses_c2r_rows(p))
         return p.k->fn_c2r;
     const TileArgs &a = p.a;
+    const TileFlavours &fl = p.k->fl;
+    const bool plain = a.epilogue == EPI_PLAIN, r2c = a.epilogue == EPI_R2C;
+    const bool byrow = a.epilogue == EPI_TWIDDLE && a.tw_by_y;
+    const bool colpow = a.epilogue == EPI_TWIDDLE && !a.tw_by_y && a.tw_colpow;
     const void *f = nullptr;
-    if (a.prologue == PRO_PLAIN && !a.half) {
-        if (a.epilogue == EPI_PLAIN)
-            f = p.k->fl.plain;
-        else if (a.epilogue == EPI_R2C)
-            f = p.k->fl.r2c;
-        else if (a.epilogue == EPI_TWIDDLE && a.tw_by_y)
-            f = p.k->fl.byrow;
-        else if (a.epilogue == EPI_TWIDDLE && a.tw_colpow)
-            f = p.k->fl.colpow;
-    }
+    if (a.prologue == PRO_PLAIN && !a.half)
+        f = plain ? fl.plain : (r2c ? fl.r2c : (byrow ? fl.byrow : (colpow ? fl.colpow : nullptr)));
+    else if (a.prologue == PRO_PLAIN)
+        f = plain ? fl.half_plain : (r2c ? fl.half_r2c : (colpow ? fl.half_colpow : nullptr));
+    else if (a.half)
+        f = nullptr;
+    else if (a.prologue == PRO_MUL)
+        f = plain ? fl.mul_plain : (colpow ? fl.mul_colpow : nullptr);
+    else if (colpow)
+        f = a.prologue == PRO_C2R ? fl.c2r_colpow : fl.mul_c2r_colpow;
     return f ? f : p.k->fn;
 }
 

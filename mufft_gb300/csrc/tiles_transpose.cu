@@ -1,41 +1,33 @@
 // Row passes with transposed stores (second pass of the four-step FFT): loads
 // walk along each row, stores walk across neighbouring rows.
-#include "fft_device.cuh"
-#include "registry.h"
+#include "tile_table.cuh"
 
 namespace mgb {
 
-#define TILE_Q(L, R, C, Q)                                                                            \
-    out.push_back(TileKernel{L, R, C, Q, ALONG, ACROSS, (const void *)&tile_fft<L, R, C, Q, ALONG, ACROSS>, \
-                             C *(L / (R * Q)), tile_smem_bytes<L, R, C, Q, ALONG, ACROSS>(),                \
-                             tile_has_thi<L, R, C, Q, ALONG, ACROSS>(), tile_exchange_bytes<L, R, C, Q, ALONG, ACROSS>(), \
-                             tile_flavours<L, R, C, Q, ALONG, ACROSS>()})
-#define TILE(L, R, C) TILE_Q(L, R, C, 1)
-
 void register_tiles_transpose(std::vector<TileKernel> &out)
 {
-    TILE(32, 16, 128);
-    TILE(64, 16, 64);
-    TILE(128, 16, 32);
-    TILE(256, 16, 16);
-    TILE(256, 16, 32);
-    TILE(512, 16, 8);
-    TILE(1024, 16, 8);
-    TILE(1024, 16, 16);
-    TILE(2048, 16, 4);
-    TILE(2048, 16, 8);
-    TILE(4096, 16, 4);       // default: measured fastest for the 4096 x 4096 four-step
-    TILE_Q(4096, 16, 4, 4);  // the same tile spread over a 4-CTA cluster
-    TILE(4096, 16, 2);
-    TILE(4096, 32, 4);
-    TILE(4096, 32, 2);
-    TILE(8192, 32, 2);
-    TILE(16384, 32, 1);
+    add_tile<32, 16, 128, 1, ALONG, ACROSS>(out);
+    add_tile<64, 16, 64, 1, ALONG, ACROSS>(out);
+    add_tile<128, 16, 32, 1, ALONG, ACROSS>(out);
+    add_tile<256, 16, 16, 1, ALONG, ACROSS>(out);
+    add_tile<256, 16, 32, 1, ALONG, ACROSS>(out);
+    add_tile<512, 16, 8, 1, ALONG, ACROSS>(out);
+    add_tile<1024, 16, 8, 1, ALONG, ACROSS>(out);
+    add_tile<1024, 16, 16, 1, ALONG, ACROSS>(out);
+    add_tile<2048, 16, 4, 1, ALONG, ACROSS>(out);
+    add_tile<2048, 16, 8, 1, ALONG, ACROSS>(out);
+    add_tile<4096, 16, 4, 1, ALONG, ACROSS>(out);       // default: measured fastest for the 4096 x 4096 four-step
+    add_tile<4096, 16, 4, 4, ALONG, ACROSS>(out);  // the same tile spread over a 4-CTA cluster
+    add_tile<4096, 16, 2, 1, ALONG, ACROSS>(out);
+    add_tile<4096, 32, 4, 1, ALONG, ACROSS>(out);
+    add_tile<4096, 32, 2, 1, ALONG, ACROSS>(out);
+    add_tile<8192, 32, 2, 1, ALONG, ACROSS>(out);
+    add_tile<16384, 32, 1, 1, ALONG, ACROSS>(out);
     // further shapes, chosen by size (choose_tile)
-    TILE(256, 16, 8);
-    TILE(512, 32, 8);
-    TILE(1024, 32, 8);
-    TILE(2048, 32, 4);
+    add_tile<256, 16, 8, 1, ALONG, ACROSS>(out);
+    add_tile<512, 32, 8, 1, ALONG, ACROSS>(out);
+    add_tile<1024, 32, 8, 1, ALONG, ACROSS>(out);
+    add_tile<2048, 32, 4, 1, ALONG, ACROSS>(out);
 }
 
 }  // namespace mgb
