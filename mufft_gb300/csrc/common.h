@@ -86,9 +86,6 @@ struct TileArgs {
     long long mirror_ldist;   // see tile kernel: local index = t*ldist + n*stride
     // convolution prologues
     const float2 *in2;        // second spectrum (B)
-    // multiply epilogue (class pipelines): output k of transform t times
-    // scale * in2[t*in2_dist + k*in2_stride]
-    long long in2_dist, in2_stride;
     // per-transform buffers (tile_body with TAB): transform t reads in_tab[t]
     // (and in2_tab[t]) and writes out_tab[t]; in_dist / out_dist are then 0
     const float2 *const *in_tab;

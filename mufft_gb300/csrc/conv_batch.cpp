@@ -72,61 +72,36 @@ void destroy_conv_batch(mufft_gb_conv_batch *b)
 
 // Task list for a split size, uploaded with the request table, and the graph
 // (counter resets + the persistent launch) that replays it.
-// Launches of one class pipeline (five four-step phases over the class's
-// requests) on `st`.
+// Launches of one class pipeline on `st`.
 bool enqueue_class(mufft_gb_conv_batch *b, unsigned lg, bool stereo, bool zp, const ClassEntry *tab, unsigned K,
                    cudaStream_t st)
 {
-    const int L1 = lg == 16 ? 256 : 128, L2 = lg == 14 ? 128 : 256, L = L1 * L2;
-    const ClassTile ct = class_column_tile(L1), rt = class_row_tile(L2), rmt = class_row_mul_tile(L2);
-    TileArgs base{};
-    base.tw = g_dev[b->device].tw;
-    base.scale = 1.0f;
-    base.tw_scale = 2.0f / (float)L;
-    base.tw_mask = (unsigned)(L - 1);
-    TileArgs cols = base, rows = base;
+    unsigned L1 = lg == 16 ? 256 : 128;
+    const unsigned L2 = lg == 14 ? 128 : 256, L = L1 * L2;
+    TileArgs cols{};
+    cols.tw = g_dev[b->device].tw;
+    cols.scale = 1.0f;
+    cols.tw_scale = 2.0f / (float)L;
+    cols.tw_mask = L - 1;
     cols.in_stride = cols.out_stride = L2;
     cols.in_dist = cols.out_dist = 1;
-    cols.ntrans = (unsigned)L2;
-    rows.in_stride = rows.out_stride = 1;
-    rows.in_dist = rows.out_dist = L2;
-    rows.ntrans = (unsigned)L1;
-    TileArgs ph[5] = {cols, rows, base, rows, cols};
-    ph[0].half = zp ? 1 : 0;
-    ph[0].epilogue = EPI_TWIDDLE;
-    ph[0].tw_colpow = 1;
-    ph[3].conj = 1;
-    ph[3].epilogue = EPI_TWIDDLE;
-    ph[4].conj = 2;
-    if (stereo) {
-        // the spectral multiply rides in F2's epilogue: X[k1 + L1*k2] * H[k1 + L1*k2] / L
-        ph[1].in2_dist = 1;
-        ph[1].in2_stride = L1;
-        ph[1].scale = 1.0f / (float)L;
-    }
-    for (int phase = 0; phase < 5; phase++) {
-        cudaError_t e;
-        if (phase == 2 && stereo)
-            continue;
-        if (phase == 2) {
-            // mono: r2c pairs, multiply, c2r pairs (stereo classes did it in F2)
-            const unsigned l1 = ilog2u((unsigned)L1), l2 = ilog2u((unsigned)L2);
-            float scale = 1.0f / (float)(2 * L);
-            const float2 *rf = b->d_rtw + b->args.rtw_off[lg], *ri = rf + L;
-            void *args[] = {(void *)&tab, (void *)&l1, (void *)&l2, &scale, (void *)&rf, (void *)&ri};
-            e = cudaLaunchKernel(class_multiply_fn(), dim3((unsigned)(L1 / 32), (unsigned)(L2 / 64), K), dim3(256), args,
-                                 0, st);
-        } else {
-            const ClassTile &t = (phase == 0 || phase == 4) ? ct : (phase == 1 && stereo ? rmt : rt);
-            const unsigned tiles = (phase == 0 || phase == 4) ? (unsigned)(L2 / t.C) : (unsigned)(L1 / t.C);
-            int phase_ = phase;
-            void *args[] = {&ph[phase], (void *)&tab, &phase_};
-            e = cudaLaunchKernel(t.fn, dim3(tiles, K), dim3(t.threads), args, t.smem, st);
-        }
-        if (!cuda_ok(e, "class launch"))
-            return false;
-    }
-    return true;
+    cols.ntrans = L2;
+    TileArgs last = cols;
+    cols.half = zp ? 1 : 0;
+    cols.epilogue = EPI_TWIDDLE;
+    cols.tw_colpow = 1;
+    last.conj = 2;  // I2: inverse over k1 of conj(Z), conjugated out
+    const ClassTile f1 = class_column_tile((int)L1, true, zp), rows = class_row_tile((int)L2, !stereo),
+                    i2 = class_column_tile((int)L1, false, false);
+    void *a1[] = {&cols, (void *)&tab};
+    float scale = 1.0f / (float)(stereo ? L : 2 * L);
+    const float2 *tw = g_dev[b->device].tw, *rtw = b->d_rtw + b->args.rtw_off[lg];
+    void *ar[] = {(void *)&tab, &L1, &scale, (void *)&tw, (void *)&rtw};
+    void *a2[] = {&last, (void *)&tab};
+    return cuda_ok(cudaLaunchKernel(f1.fn, dim3(L2 / f1.C, K), dim3(f1.threads), a1, f1.smem, st), "class launch") &&
+           cuda_ok(cudaLaunchKernel(rows.fn, dim3(L1 / rows.C, K), dim3(rows.threads), ar, rows.smem, st),
+                   "class launch") &&
+           cuda_ok(cudaLaunchKernel(i2.fn, dim3(L2 / i2.C, K), dim3(i2.threads), a2, i2.smem, st), "class launch");
 }
 
 bool conv_batch_build(mufft_gb_conv_batch *b, unsigned split_lg, unsigned class_lg, unsigned small_grid)

@@ -41,6 +41,36 @@ constexpr int kThreads = 512;
 template <int L> __host__ __device__ constexpr int single_r() { return L > 8192 ? 32 : 16; }
 template <int L> __host__ __device__ constexpr int single_c() { return kThreads * single_r<L>() / L; }
 
+// The two tiles of a whole request (or a group of them: TAB), each compiled
+// for its form.
+template <int L, int R, int C, bool TAB, int FL, bool COH>
+__device__ __forceinline__ void conv_tile(const TileArgs &a, float2 *smem)
+{
+    tile_body<L, R, C, 1, ALONG, ALONG, COH, false, false, false, TAB, FL>(a, 0, 0, 0, 0, smem);
+}
+
+template <int L, int R, int C, bool TAB>
+__device__ __forceinline__ void conv_forward(const TileArgs &f, bool mono, float2 *smem)
+{
+    if (mono && f.half)
+        conv_tile<L, R, C, TAB, FL_HALF_R2C, false>(f, smem);
+    else if (mono)
+        conv_tile<L, R, C, TAB, FL_R2C, false>(f, smem);
+    else if (f.half)
+        conv_tile<L, R, C, TAB, FL_HALF_PLAIN, false>(f, smem);
+    else
+        conv_tile<L, R, C, TAB, FL_PLAIN, false>(f, smem);
+}
+
+template <int L, int R, int C, bool TAB>
+__device__ __forceinline__ void conv_inverse(const TileArgs &b, bool mono, float2 *smem)
+{
+    if (mono)
+        conv_tile<L, R, C, TAB, FL_MUL_C2R_PLAIN, true>(b, smem);
+    else
+        conv_tile<L, R, C, TAB, FL_MUL_PLAIN, true>(b, smem);
+}
+
 // Forward tile into the spectrum scratch, then the fused multiply + inverse
 // tile into the output.
 template <int L>
@@ -60,7 +90,7 @@ __device__ void conv_single(const RaggedReq &q, float2 *smem, const float2 *tw, 
     f.tw = tw;
     f.rtw = rtw_fwd;
     f.scale = 1.0f;
-    tile_body<L, R, C, 1, ALONG, ALONG, false>(f, 0, 0, 0, 0, smem);
+    conv_forward<L, R, C, false>(f, mono, smem);
     __syncthreads();  // spectrum complete and visible to the whole CTA
 
     TileArgs b{};
@@ -76,7 +106,7 @@ __device__ void conv_single(const RaggedReq &q, float2 *smem, const float2 *tw, 
     b.scale = q.scale;
     b.conj = 3;
     b.tw = tw;
-    tile_body<L, R, C, 1, ALONG, ALONG, true>(b, 0, 0, 0, 0, smem);
+    conv_inverse<L, R, C, false>(b, mono, smem);
     __syncthreads();
 }
 
@@ -102,7 +132,7 @@ __device__ void conv_group(const RaggedReq &q, const float2 *const *tab, unsigne
     f.tw = tw;
     f.rtw = rtw_fwd;
     f.scale = 1.0f;
-    tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, false, true>(f, 0, 0, 0, 0, smem);
+    conv_forward<L, R, C, true>(f, mono, smem);
     __syncthreads();  // spectra complete and visible to the whole CTA
 
     TileArgs b{};
@@ -120,7 +150,7 @@ __device__ void conv_group(const RaggedReq &q, const float2 *const *tab, unsigne
     b.scale = q.scale;
     b.conj = 3;
     b.tw = tw;
-    tile_body<L, R, C, 1, ALONG, ALONG, true, false, false, false, false, true>(b, 0, 0, 0, 0, smem);
+    conv_inverse<L, R, C, true>(b, mono, smem);
     __syncthreads();
 }
 
@@ -388,128 +418,156 @@ size_t conv_ragged_smem()
 
 namespace {
 
-// Phase launches of class pipelines (see conv_ragged.h): F1 reads the request's
-// input, I2 writes its output, the others work on its spectrum scratch.
-template <int L, int C, int LMAP, int SMAP>
+// Column passes of class pipelines (see conv_ragged.h): F1 reads the request's
+// input (FL: with the twiddle, zero-padded or whole), I2 (FL_PLAIN) writes its
+// output; the spectrum scratch is the other side.
+template <int L, int C, int FL>
 __global__ void __launch_bounds__(tile_threads<L, 16, C, 1>(), tile_min_blocks<L, 16, C, 1>())
-    class_tile(const TileArgs tmpl, const ClassEntry *tab, int phase)
+    class_columns(const TileArgs tmpl, const ClassEntry *tab)
 {
     extern __shared__ float2 smem[];
     const ClassEntry e = tab[blockIdx.y];
     TileArgs a = tmpl;
-    a.in = phase == 0 ? e.in : e.spec;
-    a.out = phase == 4 ? e.out : e.spec;
-    tile_body<L, 16, C, 1, LMAP, SMAP, false>(a, blockIdx.x, 0, 0, 0, smem);
+    a.in = FL == FL_PLAIN ? e.spec : e.in;
+    a.out = FL == FL_PLAIN ? e.out : e.spec;
+    tile_body<L, 16, C, 1, ACROSS, ACROSS, false, false, false, false, false, FL>(a, blockIdx.x, 0, 0, 0, smem);
 }
 
-// Phase 1 of a stereo class with the spectral multiply fused into its
-// epilogue: rows k1 of X^T[k1][k2] = X[k1 + L1*k2], times s * H[k1 + L1*k2]
-// (the template's in2_dist = 1, in2_stride = L1); the multiply launch is
-// skipped.  Neighbouring rows of a tile read H's neighbouring elements.
-template <int L, int C>
-__global__ void __launch_bounds__(tile_threads<L, 16, C, 1>(), tile_min_blocks<L, 16, C, 1>())
-    class_tile_mul(const TileArgs tmpl, const ClassEntry *tab, int phase)
+// The rows of a class pipeline in one pass over the scratch: forward row
+// transforms of C rows (F2), the spectral multiply and the inverse ones with
+// the W_L^(n2*k1) twiddle (I1).  Row k1 of the scratch holds X^T[k1][k2] =
+// X[k1 + L1*k2]; the forward tile's last stage leaves positions tl + TL*j of a
+// row in registers, which is what the inverse tile's first stage wants, so
+// the spectrum itself never leaves them.  There the threads walk across the
+// tile's rows, so the filter spectrum and the fix-up twiddles, indexed by k =
+// k1 + L1*k2, are read along k1.
+//   stereo: X[k] * H[k].
+//   mono: the packed reals' spectrum Z pairs k with L - k, which sits in row
+//     L1 - k1 at column L2 - 1 - k2 (row 0: row 0, L2 - k2): a tile takes C / 2
+//     rows and their mirror rows (row 0 beside row L1 / 2, its own mirror), and
+//     the threads exchange Z through shared memory once more.  X[k] and X[L-k]
+//     come from one fix-up (r2c_bins), then the products, then the c2r one.
+// Against three launches (stereo two) with the spectrum through L2 between
+// them the 512-request mix takes 66.2 us instead of 86.9, 200 requests of 2^7
+// .. 2^15 27.6 instead of 40.2.  Bound by latency: a class is a few hundred CTAs.
+template <int L2, int C, bool MONO>
+__global__ void __launch_bounds__(256, 3)
+    class_rows(const ClassEntry *tab, unsigned L1, float scale, const float2 *tw, const float2 *rtw)
 {
+    using S = Sched<L2, 16>;
+    constexpr int R = 16, TL = L2 / R, NST = S::NST, rl = S::radix(NST - 1), NBL = R / rl, PS = S::PS;
+    constexpr int RS = region_stride<L2, C, true, PS>();
+    static_assert(TL * C == 256 && NST > 1, "256-thread row tile");
     extern __shared__ float2 smem[];
+    float2 *thi = smem + C * RS;
     const ClassEntry e = tab[blockIdx.y];
-    TileArgs a = tmpl;
-    a.in = e.spec;
-    a.out = e.spec;
-    a.in2 = e.h;
-    (void)phase;
-    tile_body<L, 16, C, 1, ALONG, ALONG, false, false, false, false, true>(a, blockIdx.x, 0, 0, 0, smem);
-}
-
-// The multiply phase of a mono class (stereo classes fuse it into F2), on the
-// transposed spectrum X^T[k1][k2] = X[k1 + L1*k2] of the packed reals (as
-// conv_multiply above): the r2c pair X[k], X[L-k] sits in rows k1 and L1-k1
-// (row 0 pairs with itself, column L2-k2).  A CTA takes 32 rows x 32 columns
-// of the lower half (k2 < L2/2, i.e. k < L/2) of request blockIdx.z and the
-// mirror elements, staged in shared memory by row-contiguous loads; the
-// filter spectrum and the twiddle tables, indexed by k, are then read along
-// k1 -- contiguously too.  k = 0 (paired with X[L]) and the self-mirrored
-// k = L/2 (row 0, column L2/2) are the special cases.
-__global__ void __launch_bounds__(256) class_multiply(const ClassEntry *tab, unsigned l1, unsigned l2, float scale,
-                                                      const float2 *rtw_fwd, const float2 *rtw_inv)
-{
-    __shared__ float2 lo[32][33], hi[32][33];
-    const ClassEntry e = tab[blockIdx.z];
-    const int L1 = 1 << l1, L2 = 1 << l2, L = L1 * L2;
-    float2 *s = e.spec;
-    const int a = blockIdx.x * 32, b = blockIdx.y * 32;
-    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    auto mirror = [&](int k1, int k2) { return k1 == 0 ? ((L2 - k2) & (L2 - 1)) : (L1 - k1) * L2 + (L2 - 1 - k2); };
-    for (int i = w; i < 32; i += 8) {
-        lo[i][lane] = s[(a + i) * L2 + b + lane];
-        hi[i][lane] = s[mirror(a + i, b + lane)];
+    const unsigned L = L1 * L2;
+    // row of the tile's transform c
+    auto row_of = [&](int c) -> unsigned {
+        if (!MONO)
+            return blockIdx.x * C + c;
+        const unsigned lo = blockIdx.x * (C / 2) + (c & (C / 2 - 1));
+        return c < C / 2 ? lo : (lo == 0 ? L1 / 2 : L1 - lo);
+    };
+    float2 v[R];
+    int c, tl;
+    split_tid<ALONG, C, TL>(threadIdx.x, c, tl);
+    const float2 *in = e.spec + (size_t)row_of(c) * L2 + tl;
+#pragma unroll
+    for (int m = 0; m < R; m++)
+        v[m] = ld_data(in + TL * m);
+    // the inverse's twiddle while the loads are in flight: W_L^(row * off) for
+    // the R output offsets of each row, and this thread's W_L^(row * tl)
+    const float tws = 2.0f / (float)L;
+    for (int idx = threadIdx.x; idx < C * R; idx += 256) {
+        const int i = idx / C;
+        thi[idx] = fourstep_twiddle(row_of(idx % C) * (unsigned)(TL * (i / rl) + (i % rl) * (L2 / rl)), tws, L - 1);
     }
-    __syncthreads();
-    for (int jj = w; jj < 32; jj += 8) {
-        const int k = a + lane + L1 * (b + jj);
-        if (k == 0) {
-            // s[0] holds Z[0]: X[0] and X[L] from its real and imaginary parts
-            const float2 z0 = lo[lane][jj];
-            const float2 x0 = make_float2(z0.x + z0.y, 0.f), xm = make_float2(z0.x - z0.y, 0.f);
-            const float2 y0 = cscale(cmul(x0, __ldg(&e.h[0])), scale);
-            const float2 ym = cscale(cmul(xm, __ldg(&e.h[L])), scale);
-            lo[lane][jj] = hi[lane][jj] = c2r_fixup(y0, ym, __ldg(&rtw_inv[0]));  // both name s[0]
-            continue;
+    const float2 wbase = fourstep_twiddle(row_of(c) * (unsigned)tl, tws, L - 1);
+    stage_compute<L2, R, 1, 0>(v, 0, tl, tw);
+    run_stages<L2, R, C, 1, ALONG, ACROSS, 1>(v, 0, c, tl, smem, tw);
+    // register u*rl + m holds position tl + TL*(u + NBL*m): in order of position
+    float2 z[R];
+#pragma unroll
+    for (int j = 0; j < R; j++)
+        z[j] = v[(j % NBL) * rl + j / NBL];
+    const unsigned k1 = row_of(c);
+    const float2 *h = e.h + k1 + (size_t)L1 * tl;
+    const size_t hstep = (size_t)L1 * TL;
+    __syncthreads();  // every thread has read its last stage's inputs
+    if constexpr (MONO) {
+        float2 *mine = smem + c * RS;
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            mine[padpos<PS>(tl + TL * j)] = z[j];
+        __syncthreads();
+        const bool self = k1 == 0 || k1 == L1 / 2;
+        const float2 *theirs = smem + (self ? c : c ^ (C / 2)) * RS;
+        const float2 *w = rtw + k1 + (size_t)L1 * tl;
+        const float2 *hm = e.h + (L - k1 - (size_t)L1 * tl);
+#pragma unroll
+        for (int j = 0; j < R; j++) {
+            const int pos = tl + TL * j;
+            const int mp = k1 == 0 ? ((L2 - pos) & (L2 - 1)) : L2 - 1 - pos;
+            const float2 zm = theirs[padpos<PS>(mp)];
+            const float2 wf = __ldg(w + hstep * j);
+            float2 xk, xm;
+            if (k1 == 0 && pos == 0) {  // X[0] and X[L] from one value
+                xk = make_float2(z[j].x + z[j].y, 0.f);
+                xm = make_float2(z[j].x - z[j].y, 0.f);
+            } else {
+                r2c_bins(z[j], zm, wf, xk, xm);
+                xm = cconj(xm);
+            }
+            const float2 yk = cscale(cmul(xk, ld_data(h + hstep * j)), scale);
+            const float2 ym = cscale(cmul(xm, ld_data(hm - hstep * j)), scale);
+            z[j] = cconj(c2r_fixup(yk, ym, cconj(wf)));  // the c2r twiddle is the r2c one's conjugate
         }
-        const int km = L - k;
-        const float2 zk = lo[lane][jj], zm = hi[lane][jj];
-        float2 xk, xk_hi, xm, xm_hi;
-        r2c_bins(zk, zm, __ldg(&rtw_fwd[k]), xk, xk_hi);
-        r2c_bins(zm, zk, __ldg(&rtw_fwd[km]), xm, xm_hi);
-        const float2 yk = cscale(cmul(xk, __ldg(&e.h[k])), scale);
-        const float2 ym = cscale(cmul(xm, __ldg(&e.h[km])), scale);
-        lo[lane][jj] = c2r_fixup(yk, ym, __ldg(&rtw_inv[k]));
-        hi[lane][jj] = c2r_fixup(ym, yk, __ldg(&rtw_inv[km]));
+        __syncthreads();  // the slices are free again
+    } else {
+#pragma unroll
+        for (int j = 0; j < R; j++)
+            z[j] = cconj(cscale(cmul(z[j], ld_data(h + hstep * j)), scale));
     }
-    __syncthreads();
-    for (int i = w; i < 32; i += 8) {
-        s[(a + i) * L2 + b + lane] = lo[i][lane];
-        s[mirror(a + i, b + lane)] = hi[i][lane];
-    }
-    if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0) {
-        const int k = L / 2, idx = L2 / 2;  // row 0, column L2/2: X[L/2] pairs with itself
-        const float2 zk = s[idx];
-        float2 xk, xk_hi;
-        r2c_bins(zk, zk, __ldg(&rtw_fwd[k]), xk, xk_hi);
-        const float2 yk = cscale(cmul(xk, __ldg(&e.h[k])), scale);
-        s[idx] = c2r_fixup(yk, yk, __ldg(&rtw_inv[k]));
-    }
+    stage_compute<L2, R, 1, 0>(z, 0, tl, tw);
+    run_stages<L2, R, C, 1, ACROSS, ALONG, 1, true>(z, 0, c, tl, smem, tw, wbase);
+    float2 *out = e.spec + (size_t)row_of(c) * L2 + tl;
+#pragma unroll
+    for (int u = 0; u < NBL; u++)
+#pragma unroll
+        for (int m = 0; m < rl; m++)
+            out[TL * u + m * (L2 / rl)] = cmul(z[u * rl + m], thi[(u * rl + m) * C + c]);
+}
+
+template <int L2, int C> constexpr size_t class_rows_bytes()
+{
+    return ((size_t)C * region_stride<L2, C, true, Sched<L2, 16>::PS>() + (size_t)C * 16) * sizeof(float2);
+}
+
+template <int L, int C> ClassTile column_tile(int form)
+{
+    const void *fn = form == 0   ? (const void *)&class_columns<L, C, FL_COLPOW>
+                     : form == 1 ? (const void *)&class_columns<L, C, FL_HALF_COLPOW>
+                                 : (const void *)&class_columns<L, C, FL_PLAIN>;
+    return ClassTile{fn, L, C, tile_threads<L, 16, C, 1>(), tile_smem_bytes<L, 16, C, 1, ACROSS, ACROSS>()};
 }
 
 }  // namespace
 
-ClassTile class_column_tile(int L1)
+ClassTile class_column_tile(int L1, bool first, bool zero_pad)
 {
-    if (L1 == 128)
-        return ClassTile{(const void *)&class_tile<128, 32, ACROSS, ACROSS>, 128, 32, tile_threads<128, 16, 32, 1>(),
-                         tile_smem_bytes<128, 16, 32, 1, ACROSS, ACROSS>()};
-    return ClassTile{(const void *)&class_tile<256, 16, ACROSS, ACROSS>, 256, 16, tile_threads<256, 16, 16, 1>(),
-                     tile_smem_bytes<256, 16, 16, 1, ACROSS, ACROSS>()};
+    const int form = first ? (zero_pad ? 1 : 0) : 2;
+    return L1 == 128 ? column_tile<128, 32>(form) : column_tile<256, 16>(form);
 }
 
-ClassTile class_row_tile(int L2)
+ClassTile class_row_tile(int L2, bool mono)
 {
     if (L2 == 128)
-        return ClassTile{(const void *)&class_tile<128, 32, ALONG, ALONG>, 128, 32, tile_threads<128, 16, 32, 1>(),
-                         tile_smem_bytes<128, 16, 32, 1, ALONG, ALONG>()};
-    return ClassTile{(const void *)&class_tile<256, 16, ALONG, ALONG>, 256, 16, tile_threads<256, 16, 16, 1>(),
-                     tile_smem_bytes<256, 16, 16, 1, ALONG, ALONG>()};
+        return ClassTile{mono ? (const void *)&class_rows<128, 32, true> : (const void *)&class_rows<128, 32, false>, 128,
+                         32, 256, class_rows_bytes<128, 32>()};
+    return ClassTile{mono ? (const void *)&class_rows<256, 16, true> : (const void *)&class_rows<256, 16, false>, 256, 16,
+                     256, class_rows_bytes<256, 16>()};
 }
-
-ClassTile class_row_mul_tile(int L2)
-{
-    if (L2 == 128)
-        return ClassTile{(const void *)&class_tile_mul<128, 32>, 128, 32, tile_threads<128, 16, 32, 1>(),
-                         tile_smem_bytes<128, 16, 32, 1, ALONG, ALONG>()};
-    return ClassTile{(const void *)&class_tile_mul<256, 16>, 256, 16, tile_threads<256, 16, 16, 1>(),
-                     tile_smem_bytes<256, 16, 16, 1, ALONG, ALONG>()};
-}
-
-const void *class_multiply_fn() { return (const void *)&class_multiply; }
 
 const void *conv_ragged_fn() { return (const void *)&conv_ragged_kernel; }
 int conv_ragged_threads() { return kThreads; }

@@ -61,8 +61,9 @@ int conv_ragged_threads();
 size_t conv_ragged_smem();
 
 // Class pipelines: requests of one (size, method, zero-pad) class whose
-// five four-step phases run as ordinary batched launches over a table of the
-// requests' buffers (blockIdx.y picks the request).
+// four-step runs as three ordinary batched launches over a table of the
+// requests' buffers (blockIdx.y picks the request): F1 columns; F2 rows, the
+// multiply and I1 rows; I2 columns.
 struct ClassEntry {
     const float2 *in;
     const float2 *h;
@@ -71,20 +72,16 @@ struct ClassEntry {
 };
 
 struct ClassTile {
-    const void *fn;  // kernel(TileArgs tmpl, const ClassEntry *tab, int phase)
+    const void *fn;
     int L, C, threads;
     size_t smem;     // with the twiddle region
 };
-// Phase 0/4 (columns of L1) and 1/3 (rows of L2) tiles for a split L1 x L2.
-ClassTile class_column_tile(int L1);
-ClassTile class_row_tile(int L2);
-// Phase 1 with the stereo spectral multiply fused, kernel(TileArgs tmpl,
-// const ClassEntry *tab, int phase) with the template's in2_dist = 1,
-// in2_stride = L1 and scale = 1 / L; the multiply launch is then skipped.
-ClassTile class_row_mul_tile(int L2);
-// Multiply phase of a mono class: kernel(const ClassEntry *tab, unsigned l1,
-// unsigned l2, float scale, const float2 *rtw_fwd, const float2 *rtw_inv),
-// grid (L1/32, L2/64, requests), 256 threads.
-const void *class_multiply_fn();
+// First (F1, zero-padded input or not) and last (I2) pass: columns of L1,
+// kernel(TileArgs tmpl, const ClassEntry *tab), grid (L2 / C, requests).
+ClassTile class_column_tile(int L1, bool first, bool zero_pad);
+// The pass between: forward rows of L2, spectral multiply, inverse rows,
+// kernel(const ClassEntry *tab, unsigned L1, float scale, const float2 *tw,
+// const float2 *rtw_fwd), grid (L1 / C, requests).
+ClassTile class_row_tile(int L2, bool mono);
 
 }  // namespace mgb

@@ -540,6 +540,7 @@ enum Flavour : int {
     FL_HALF_R2C = form(PRO_PLAIN, 1, EPI_R2C),
     FL_HALF_COLPOW = form(PRO_PLAIN, 1, EPI_TWIDDLE, 1),
     FL_MUL_PLAIN = form(PRO_MUL, 0, EPI_PLAIN),
+    FL_MUL_C2R_PLAIN = form(PRO_MUL_C2R, 0, EPI_PLAIN),
     FL_MUL_COLPOW = form(PRO_MUL, 0, EPI_TWIDDLE, 1),
     FL_C2R_COLPOW = form(PRO_C2R, 0, EPI_TWIDDLE, 1),
     FL_MUL_C2R_COLPOW = form(PRO_MUL_C2R, 0, EPI_TWIDDLE, 1),
@@ -894,12 +895,10 @@ template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_min
 // PRE: the stage-0 registers were loaded by the caller (`pre`, R values).
 // C2RS: c2r fix-up prologue through a row staged in shared memory (row
 // tiles; the caller checked load_stage0_c2r_rows's conditions).
-// EMUL: plain epilogue multiplied by scale * in2[tr*in2_dist + k*in2_stride]
-// (the spectral multiply of a convolution, fused into the forward pass).
 // TAB: every transform of the tile has its own buffers (in_tab / in2_tab /
 // out_tab, distances 0): a tile of C unrelated requests of one size.
 template <int L, int R, int C, int Q, int LMAP, int SMAP, bool COH, bool SIN = false, bool PRE = false,
-          bool C2RS = false, bool EMUL = false, bool TAB = false, int FL = FL_ANY>
+          bool C2RS = false, bool TAB = false, int FL = FL_ANY>
 __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int j, long long ioff, long long ooff,
                                           float2 *smem, const float2 *sin = nullptr, unsigned twy = 0,
                                           const float2 *pre = nullptr)
@@ -1158,8 +1157,6 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                     float2 y = v[u * rl + m];
                     if constexpr (!std::is_same<decltype(w), std::nullptr_t>::value)
                         y = cmul(y, w(u * rl + m, TL * u + m * Q * BL));
-                    if constexpr (EMUL)
-                        y = cscale(y, a.scale);
                     st_policy(dst, sign(y), stpol);
                     dst += mstep;
                 }
@@ -1199,9 +1196,6 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
                     return fourstep_twiddle((unsigned)(p0 + off) * col, a.tw_scale, a.tw_mask);
                 });
             }
-        } else if constexpr (EMUL) {
-            const float2 *e = a.in2 + (long long)tr * a.in2_dist + (long long)p0 * a.in2_stride;
-            emit([&](int, int off) { return ld_data(e + (long long)off * a.in2_stride); });
         } else {
             emit(nullptr);
         }
@@ -1230,8 +1224,8 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, Q>(), tile_min_blocks<L,
         j = (int)cg::this_cluster().block_rank();
         tile = blockIdx.x / Q;
     }
-    tile_body<L, R, C, Q, LMAP, SMAP, false, false, false, false, false, false, FL>(a, tile, j, ioff, ooff, smem, nullptr,
-                                                                                   blockIdx.y);
+    tile_body<L, R, C, Q, LMAP, SMAP, false, false, false, false, false, FL>(a, tile, j, ioff, ooff, smem, nullptr,
+                                                                            blockIdx.y);
 }
 
 // Row tile whose c2r fix-up prologue stages each row in shared memory
@@ -1252,8 +1246,7 @@ __global__ void __launch_bounds__(tile_threads<L, R, C, 1>(), tile_min_blocks<L,
         ioff = (long long)blockIdx.y * a.in_batch;
         ooff = (long long)blockIdx.y * a.out_batch;
     }
-    tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, true, false, false, FL_PLAIN>(a, blockIdx.x, 0, ioff, ooff,
-                                                                                           smem);
+    tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, true, false, FL_PLAIN>(a, blockIdx.x, 0, ioff, ooff, smem);
 }
 
 // The staged-c2r variant of a row tile, or null where there is none.

@@ -89,11 +89,11 @@ __device__ void fr_group(const FftRaggedReq &q, const float2 *const *tab, unsign
         a.mirror_len = L;
     }
     if (q.kind == FR_C2C && !q.half)
-        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, false, true, FL_PLAIN>(a, 0, 0, 0, 0, smem);
+        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, true, FL_PLAIN>(a, 0, 0, 0, 0, smem);
     else if (q.kind == FR_R2C && !q.half && !q.full)
-        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, false, true, FL_R2C>(a, 0, 0, 0, 0, smem);
+        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, true, FL_R2C>(a, 0, 0, 0, 0, smem);
     else
-        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, false, true>(a, 0, 0, 0, 0, smem);
+        tile_body<L, R, C, 1, ALONG, ALONG, false, false, false, false, true>(a, 0, 0, 0, 0, smem);
     __syncthreads();
 }
 
@@ -152,7 +152,7 @@ __device__ void fr_rows(const FftRaggedReq &q, float2 *smem, const float2 *tw, i
     a.conj = (q.kind == FR_C2R || (q.kind == FR_C2C && q.inverse)) ? 2 : 0;
     const int t0 = index < 0 ? 0 : index, t1 = index < 0 ? L1 / C2 : index + 1;
     for (int t = t0; t < t1; t++) {
-        tile_body<L2, 16, C2, 1, ALONG, ACROSS, true, false, false, false, false, false, FL_PLAIN>(a, t, 0, 0, 0, smem);
+        tile_body<L2, 16, C2, 1, ALONG, ACROSS, true, false, false, false, false, FL_PLAIN>(a, t, 0, 0, 0, smem);
         __syncthreads();
     }
 }

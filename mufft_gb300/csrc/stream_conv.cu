@@ -103,11 +103,9 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
 
     if (blockIdx.x == 0) {
         if (a.inv_c2r_rows)
-            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, false, FL_R2C>(a.fwd, 0, 0, 0, 0,
-                                                                                                  smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, FL_R2C>(a.fwd, 0, 0, 0, 0, smem);
         else
-            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, false, FL_PLAIN>(a.fwd, 0, 0, 0, 0,
-                                                                                                    smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, false, false, false, false, false, FL_PLAIN>(a.fwd, 0, 0, 0, 0, smem);
         __syncthreads();  // the spectrum is written and the whole window has been read
         if (threadIdx.x == 0)
             st_release(&a.tickets[2], k + 1);
@@ -200,10 +198,9 @@ __global__ void __launch_bounds__(256) upols_block(const UpolsBlockArgs a)
     if (flag) {
         // every group is finished: y is complete (L2-coherent loads)
         if (a.inv_c2r_rows)
-            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, true, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0, smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, true, false, FL_PLAIN>(a.inv, 0, 0, 0, 0, smem);
         else
-            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, false, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0,
-                                                                                                   smem);
+            tile_body<M, 16, C, 1, ALONG, ALONG, true, false, false, false, false, FL_PLAIN>(a.inv, 0, 0, 0, 0, smem);
         if (threadIdx.x == 0) {
             a.tickets[1] = 0;  // read again by the next launch only
             a.tickets[0] = k + 1;
