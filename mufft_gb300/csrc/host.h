@@ -30,6 +30,7 @@
 #include "registry.h"
 #include "split_tc.h"
 #include "tiles_persist.h"
+#include "tiles_r2c_rows.h"
 #include "tiles_stream.h"
 #include "tiles_tma.h"
 
@@ -65,6 +66,7 @@ const std::vector<TileKernel> &tile_table();
 const TmaTileKernel *find_tma(int L, int R, int C, int nbuf);
 const StreamTileKernel *find_stream(int L, int R, int C);
 const PersistTileKernel *find_persist(int L, int R, int C, int lmap, int smap);
+const std::vector<R2cRowsKernel> &r2c_rows_table();
 
 // ----------------------------------------------------------------- options
 
@@ -158,6 +160,9 @@ struct Pass {
     // as one launch per tile
     const PersistTileKernel *pt = nullptr;
     unsigned pt_grid = 0;
+    // second pass of a four-step r2c with the fix-up in its stores
+    // (tiles_r2c_rows.cu); `k` is the plain row tile of its length
+    const R2cRowsKernel *rk = nullptr;
 };
 
 struct Buffers {

@@ -121,6 +121,16 @@ const PersistTileKernel *find_persist(int L, int R, int C, int lmap, int smap)
     return nullptr;
 }
 
+const std::vector<R2cRowsKernel> &r2c_rows_table()
+{
+    static const std::vector<R2cRowsKernel> t = [] {
+        std::vector<R2cRowsKernel> v;
+        register_tiles_r2c_rows(v);
+        return v;
+    }();
+    return t;
+}
+
 const TileKernel *find_tile(int L, int lmap, int smap, int C, int R, int Q)
 {
     if (C == 0 && R == 0 && Q == 0 && t_opts) {

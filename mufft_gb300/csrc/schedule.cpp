@@ -13,6 +13,8 @@
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
+#include <mutex>
+#include <set>
 
 #include "host.h"
 #include "launch.h"
@@ -91,6 +93,26 @@ const TileKernel *choose_tile(int L, int lmap, int smap, unsigned long long ntra
         if (const TileKernel *t = find_tile(L, lmap, smap, 1, 32, 1))
             return t;
     return k;
+}
+
+// The row pass of a four-step r2c, N1 rows of N2 points, that resolves the
+// bins itself; null where there is none or the plan's options prefer a row
+// tile.  The 16-row tile where it gives two CTAs per SM, else the 8-row one
+// (r2c 2^18 x 1: 16 tiles of 16 rows).
+static const R2cRowsKernel *choose_r2c_rows(unsigned N1, unsigned N2, unsigned batch)
+{
+    if (t_opts)
+        for (const TileKernel &t : t_opts->tiles)
+            if (t.L == (int)N2 && t.lmap == ALONG && t.smap == ACROSS)
+                return nullptr;
+    const R2cRowsKernel *found = nullptr;
+    for (const R2cRowsKernel &k : r2c_rows_table())
+        if (k.L == (int)N2 && N1 % k.C == 0) {
+            found = &k;
+            if ((unsigned long long)(N1 / k.C) * batch >= kFill)
+                break;
+        }
+    return found;
 }
 
 static const void *pick(Role r, const Buffers &b)
@@ -197,13 +219,23 @@ static const void *tile_fn(const Pass &p)
 
 bool prepare_tile_fns(const std::vector<Pass> &ps, int device)
 {
-    int limit = 232448;
-    cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
-    for (const Pass &p : ps)
-        if (p.type == PASS_TILE && p.k && tile_launch_smem(p) > 48 * 1024 &&
-            !cuda_ok(cudaFuncSetAttribute(tile_fn(p), cudaFuncAttributeMaxDynamicSharedMemorySize, limit),
+    // each kernel once per device (the call takes 10-20 us)
+    static std::mutex mu;
+    static std::set<std::pair<int, const void *>> done;
+    for (const Pass &p : ps) {
+        if (p.type != PASS_TILE || !p.k || (p.rk ? p.rk->smem : tile_launch_smem(p)) <= 48 * 1024)
+            continue;
+        const std::pair<int, const void *> key(device, p.rk ? p.rk->fn : tile_fn(p));
+        std::lock_guard<std::mutex> lock(mu);
+        if (done.count(key))
+            continue;
+        int limit = 232448;
+        cudaDeviceGetAttribute(&limit, cudaDevAttrMaxSharedMemoryPerBlockOptin, device);
+        if (!cuda_ok(cudaFuncSetAttribute(key.second, cudaFuncAttributeMaxDynamicSharedMemorySize, limit),
                      "cudaFuncSetAttribute(tile)"))
             return false;
+        done.insert(key);
+    }
     return true;
 }
 
@@ -250,6 +282,12 @@ cudaError_t run_passes(const std::vector<Pass> &ps, const Buffers &b, cudaStream
                 continue;
             }
             void *args[] = {&a};
+            if (p.rk) {
+                cudaError_t e = launch_dependent(p.rk->fn, p.grid, dim3(p.rk->threads), args, p.rk->smem, st);
+                if (e != cudaSuccess)
+                    return e;
+                continue;
+            }
             const size_t smem = tile_launch_smem(p);
             // one tile per CTA, or per cluster of Q CTAs (distributed shared memory)
             const unsigned q = (unsigned)p.k->Q;
@@ -310,7 +348,12 @@ std::string describe(const std::vector<Pass> &ps)
     char buf[256];
     for (size_t i = 0; i < ps.size(); i++) {
         const Pass &p = ps[i];
-        if (p.type == PASS_TILE)
+        if (p.type == PASS_TILE && p.rk)
+            snprintf(buf, sizeof(buf),
+                     "%stile+r2c_rows L=%d R=%d C=%d Q=1 along/across grid=%ux%u threads=%d smem=%zu pro=plain epi=%s conj=0",
+                     i ? "; " : "", p.rk->L, p.rk->R, p.rk->C, p.grid.x, p.grid.y, p.rk->threads, p.rk->smem,
+                     epi_name(p.a.epilogue));
+        else if (p.type == PASS_TILE)
             snprintf(buf, sizeof(buf), "%stile%s L=%d R=%d C=%d Q=%d %s/%s grid=%ux%u threads=%d smem=%zu pro=%s%s epi=%s%s conj=%d",
                      i ? "; " : "", p.tk ? (p.tk->nbuf == 2 ? "+tma2" : "+tma1") : (p.sk ? "+stream" : (p.pt ? "+persistent" : "")), p.k->L, p.k->R, p.k->C, p.k->Q, p.k->lmap ? "across" : "along",
                      p.k->smap ? "across" : "along", p.sk ? p.sk_grid : (p.pt ? std::min(p.grid.x * p.grid.y, p.pt_grid) : p.grid.x), p.pt ? 1u : p.grid.y, p.k->threads, std::max(p.k->smem, p.smem_min),
@@ -483,7 +526,7 @@ bool attach_persist(std::vector<Pass> &ps, bool dry, int device)
     if (opt_persist() != 1)
         return true;
     for (Pass &p : ps) {
-        if (p.type != PASS_TILE || !p.k || p.k->Q != 1 || p.tk || p.sk || p.grid.z > 1 || uses_c2r_rows(p))
+        if (p.type != PASS_TILE || !p.k || p.k->Q != 1 || p.tk || p.sk || p.rk || p.grid.z > 1 || uses_c2r_rows(p))
             continue;
         const PersistTileKernel *pt = find_persist(p.k->L, p.k->R, p.k->C, p.k->lmap, p.k->smap);
         if (!pt)
@@ -529,7 +572,7 @@ bool attach_occupancy(std::vector<Pass> &ps, bool dry, int device)
         return true;
     const size_t want = (size_t)w & ~(size_t)127;
     for (Pass &p : ps) {
-        if (p.type != PASS_TILE || !p.k || p.k->Q != 1 || p.tk || p.sk || p.pt)
+        if (p.type != PASS_TILE || !p.k || p.k->Q != 1 || p.tk || p.sk || p.pt || p.rk)
             continue;
         if (want <= p.k->smem)
             continue;
@@ -857,6 +900,12 @@ bool build_fft_passes(const FftSpec &s, const float2 *tw, PlanResources &res, bo
     p2.in_role = ROLE_SCRATCH;
     p2.out_role = s.out_role;
     p2.grid = dim3((N1 + kr->C - 1) / kr->C, s.batch);
+    if (r2c && (p2.rk = choose_r2c_rows(N1, N2, s.batch))) {
+        p2.a.epilogue = s.epilogue;
+        p2.a.rtw = res.rtw;
+        p2.grid = dim3(N1 / p2.rk->C, s.batch);
+    }
+    const bool fixup = r2c && !p2.rk;
     if (opt_l2() == 1 && (size_t)M * s.batch * sizeof(float2) <= kL2HintMaxScratch) {
         // the intermediate as in the three-level schedule: kept in L2 by the
         // first pass, dropped without write-back once the second has read it
@@ -865,11 +914,11 @@ bool build_fft_passes(const FftSpec &s, const float2 *tw, PlanResources &res, bo
         // 917 -> 957 us, 2^20 x 128 857 -> 898 us, 2^21 x 16 246 -> 253 us)
         // against 2^16 x 256 94.2 -> 89.6 us and r2c 2^21 x 8 101.6 -> 94.0 us.
         out.back().a.l2 = L2_LOAD_FIRST | L2_STORE_LAST;
-        p2.a.l2 = L2_DISCARD_IN | (r2c ? 0 : L2_STORE_FIRST);
+        p2.a.l2 = L2_DISCARD_IN | (fixup ? 0 : L2_STORE_FIRST);
     }
     out.push_back(p2);
 
-    if (r2c) {
+    if (fixup) {
         Pass p3;
         p3.type = PASS_R2C_FIXUP;
         p3.a.rtw = res.rtw;
