@@ -285,6 +285,52 @@ mufft_plan_1d *create_1d(int kind, unsigned N, int direction, unsigned flags, un
     return pl;
 }
 
+// Where a buffer lives: memory the device owns (or migrates), or page-locked
+// host memory and its device address (null: neither).
+struct Residence {
+    bool device;
+    void *mapped;
+};
+
+static Residence residence(const void *p)
+{
+    cudaPointerAttributes at;
+    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
+        cudaGetLastError();
+        return {false, nullptr};
+    }
+    if (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged)
+        return {true, nullptr};
+    return {false, at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr};
+}
+
+// Whether a blocking execute lets the kernel read and write the caller's
+// page-locked memory itself instead of staging it: one pass, which reads and
+// writes every element once, small buffers -- a copy each way costs more than
+// the link's latency (stereo block convolution of 2048 frames, input and
+// output call: 48.0 -> 26.5 us, mono 4096 55.0 -> 28.1) -- of the kernels' alignment, and apart from
+// each other (staging also serves transforms in place).
+constexpr size_t kDirectHostBytes = (size_t)1 << 20;
+
+static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out, const void *in2,
+                        const Residence &rin, const Residence &rout, const Residence &rin2)
+{
+    if ((rin.device && rout.device && rin2.device) || pl->passes.size() != 1 || pl->passes[0].type != PASS_TILE ||
+        pl->passes[0].tk)
+        return false;
+    const size_t ib = pl->in_total(), ob = pl->out_total();
+    if (ib > kDirectHostBytes || ob > kDirectHostBytes)
+        return false;
+    for (const Residence *r : {&rin, &rout, &rin2})
+        if (!r->device && !r->mapped)
+            return false;
+    const uintptr_t i = (uintptr_t)in, o = (uintptr_t)out, i2 = (uintptr_t)in2;
+    if ((i | o | i2) & 7)
+        return false;
+    auto apart = [](uintptr_t a, size_t an, uintptr_t c, size_t cn) { return a + an <= c || c + cn <= a; };
+    return apart(i, ib, o, ob) && (!in2 || apart(i2, ib, o, ob));
+}
+
 int exec_1d(mufft_plan_1d *pl, void *out, const void *in, const void *in2, cudaStream_t st, bool sync)
 {
     if (!pl || !out || !in || (pl->uses_in2 && !in2)) {
@@ -292,9 +338,9 @@ int exec_1d(mufft_plan_1d *pl, void *out, const void *in, const void *in2, cudaS
         return MUFFT_GB_ERR_INVALID;
     }
     DeviceGuard g(pl->device);
-    const bool hin = !is_device_accessible(in);
-    const bool hin2 = pl->uses_in2 && !is_device_accessible(in2);
-    const bool hout = !is_device_accessible(out);
+    const Residence rin = residence(in), rout = residence(out),
+                    rin2 = pl->uses_in2 ? residence(in2) : Residence{true, nullptr};
+    bool hin = !rin.device, hin2 = !rin2.device, hout = !rout.device;
     if (!sync && (hin || hin2 || hout)) {
         set_error(MUFFT_GB_ERR_HOST_POINTER, "asynchronous execute needs device-accessible buffers");
         return MUFFT_GB_ERR_HOST_POINTER;
@@ -302,6 +348,12 @@ int exec_1d(mufft_plan_1d *pl, void *out, const void *in, const void *in2, cudaS
     if (sync)
         st = pl->stream;
     Buffers b{in, out, in2, pl->res.scratch};
+    if (direct_host(pl, in, out, in2, rin, rout, rin2)) {
+        b.in = rin.device ? in : rin.mapped;
+        b.out = rout.device ? out : rout.mapped;
+        b.in2 = rin2.device ? in2 : rin2.mapped;
+        hin = hin2 = hout = false;
+    }
     if (hin) {
         if (!ensure(pl->stage.in, pl->stage.in_bytes, pl->in_total()))
             return t_err;
