@@ -30,8 +30,11 @@
 // MMAs, frees TMEM, returns.
 //
 // 16384 x 4096 with three limbs: 457.8 us with the operands in shared memory (and
-// the input and output passing through it once more), 352.1 like this, bit for
-// bit the same.
+// the input and output passing through it once more), 352.1 with TMEM operands,
+// 337.8 with two exchange buffers (three barriers a block instead of seven), bit
+// for bit the same.  Bound by the chain of each stage -- limbs, products,
+// read-back -- with two CTAs of eight warps per SM: 45 % of the issue slots, the
+// tensor pipe 17 % busy.
 #include <cuda_bf16.h>
 
 #include <cmath>
@@ -53,9 +56,9 @@ constexpr unsigned kTmemA = 64;
 // shared-memory layout (bytes)
 constexpr int kInOff = 0;                          // staged input: 4096 points
 constexpr int kBOff = kInOff + 4096 * 8;           // [limb] B operands: 3 x 2 KB
-constexpr int kXOff = kBOff + 3 * 2048;            // exchange: 4096 points padded
+constexpr int kXOff = kBOff + 3 * 2048;            // two exchange buffers, 4096 points padded each
 constexpr int kXElems = 4096 + 256;                // upad(4095) + 1
-constexpr int kTwOff = kXOff + kXElems * 8;        // 512 stage twiddle factors
+constexpr int kTwOff = kXOff + 2 * kXElems * 8;        // 512 stage twiddle factors
 constexpr int kBarOff = kTwOff + 512 * 8;          // 3 mbarriers (24 B) + TMEM address (4 B)
 constexpr int kUSmem = kBarOff + 64;
 
@@ -248,29 +251,34 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
     fence_after();
     const unsigned tmem = *tmem_slot;
     unsigned phase = 0, in_phase = 0;
-    bool ok = true, in_flight = false;
+    // pending: this thread's wait for its tile's products ran out; in_flight:
+    // (thread 0) a copy of a block's input is under way
+    bool ok = true, in_flight = false, pending = false;
 
     const long long nblocks = ((long long)a.ntrans + T - 1) / T;
     if (bulk && tid == 0 && (long long)blockIdx.x < nblocks) {
         prefetch_block<N, T>(a, blockIdx.x, smem_u32(stage_in), bar_in);
         in_flight = true;
     }
-    in_flight = __syncthreads_or(in_flight) != 0;
     for (long long blk = blockIdx.x; blk < nblocks && ok; blk += gridDim.x) {
         const long long tr0 = blk * T;
+        // this thread's waits so far; all threads' are brought together at the
+        // barriers below (a thread whose wait ran out goes on to them)
+        bool good = true;
         if (bulk) {
-            ok = __syncthreads_and(tid == 0 ? bar_wait(bar_in, in_phase & 1) : true) != 0;
-            if (!ok) {
-                if (tid == 0 && a.err)
-                    atomicExch(a.err, 1);
-                break;
+            good = bar_wait(bar_in, in_phase & 1);
+            if (good) {
+                in_phase++;
+                in_flight = false;
             }
-            in_phase++;
-            in_flight = false;
         }
 
 #pragma unroll 1
         for (int s = 0; s < S && ok; s++) {
+            // the stages scatter into the two exchange buffers in turn, so a
+            // scatter never meets the gathers of its own stage
+            const float2 *from = X + (s & 1 ? 0 : kXElems);
+            float2 *to = X + (s & 1 ? kXElems : 0);
             const int p = 1 << (4 * s);
             // this thread's column: jj = tid (rows of the two M = 128 tiles)
             const int jj = tid, tt = jj / Q, j = jj % Q;
@@ -299,7 +307,7 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
             } else {
 #pragma unroll
                 for (int m = 0; m < 16; m++) {
-                    float2 v = X[upad(tt * N + j + Q * m)];
+                    float2 v = from[upad(tt * N + j + Q * m)];
                     if (s == 1)
                         v = cmul(v, t1[m * 16 + (j & 15)]);
                     else
@@ -342,29 +350,21 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
                     }
                 umma_commit(bar0 + 8 * half);
             }
-            // every gather of this stage is done before any scatter below; one
-            // thread per half waits for its tile's commit
-            ok = __syncthreads_and((tid & 127) == 0 ? bar_wait(bar0 + 8 * half, phase & 1) : true) != 0;
-            if (!ok) {
-                if (tid == 0 && a.err)
-                    atomicExch(a.err, 1);
-            } else {
+            const bool done = bar_wait(bar0 + 8 * half, phase & 1);
+            if (done)
                 phase++;
-            }
+            else
+                good = false;
+            pending = !done;
             fence_after();
-            if (ok) {
-                if (s == 0 && bulk && tid == 0 && blk + gridDim.x < nblocks) {
-                    // every thread has gathered the staged input
-                    prefetch_block<N, T>(a, blk + gridDim.x, smem_u32(stage_in), bar_in);
-                    in_flight = true;
-                }
+            if (__all_sync(0xFFFFFFFFu, done)) {
                 // D row of this thread's column: lane group (warp & 3), tile (warp >> 2)
                 float d[32];
                 tmem_ld32(tmem + lanes + (warp >> 2) * 32, d);
                 fence_before();  // before the next products of this tile (the half's barrier above)
                 if (s == S - 1) {
                     // p = Q: output k of column j is j + k*Q
-                    if (valid) {
+                    if (valid && good) {
                         float2 *dst = a.out + (tr0 + tt) * a.out_dist + j;
                         const float sg = a.conj ? -1.f : 1.f;
 #pragma unroll
@@ -375,23 +375,29 @@ __global__ void __launch_bounds__(kUThreads, 2) split_umma_fft(const SplitArgs a
 #pragma unroll
                     for (int k = 0; k < 16; k++) {
                         const int pos = tt * N + (j / p) * 16 * p + (j & (p - 1)) + k * p;
-                        X[upad(pos)] = make_float2(d[k], d[16 + k]);
+                        to[upad(pos)] = make_float2(d[k], d[16 + k]);
                     }
-                    __syncthreads();
                 }
             }
+            // the scatter is complete, or (last stage) the block is
+            ok = __syncthreads_and(good) != 0;
+            if (s == 0 && ok && bulk && tid == 0 && blk + gridDim.x < nblocks) {
+                // every thread has gathered the staged input
+                prefetch_block<N, T>(a, blk + gridDim.x, smem_u32(stage_in), bar_in);
+                in_flight = true;
+            }
         }
-        in_flight = __syncthreads_or(in_flight) != 0;
+        if (!ok && tid == 0 && a.err)
+            atomicExch(a.err, 1);
     }
     if (!ok) {
         // let this CTA's products and copies drain before TMEM is released
-        // (bounded): the timed-out phases are still `phase` / `in_phase`
-        if (tid == 0) {
-            bar_wait(bar0, phase & 1);
-            bar_wait(bar0 + 8, phase & 1);
-            if (in_flight)
-                bar_wait(bar_in, in_phase & 1);
-        }
+        // (bounded): the timed-out phases are still `phase` / `in_phase`, each
+        // half's of its own tile
+        if ((tid & 127) == 0 && pending)
+            bar_wait(bar0 + 8 * half, phase & 1);
+        if (tid == 0 && in_flight)
+            bar_wait(bar_in, in_phase & 1);
         __syncthreads();
     }
     fence_before();
