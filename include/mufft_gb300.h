@@ -264,8 +264,8 @@ typedef struct mufft_gb_conv_batch mufft_gb_conv_batch;
 /* Prepares `count` requests of mixed sizes for one persistent launch,
  * captured in a CUDA graph.  Requests of at least opts->conv_classes complex
  * points run as class pipelines: the requests of one size, method and
- * zero-pad setting go through five ordinary batched launches (the four-step
- * phases) on parallel branches of the batch's graph.  The rest run longest
+ * zero-pad setting go through three ordinary batched launches (columns; rows
+ * with the multiply; columns) on parallel branches of the batch's graph.  The rest run longest
  * first in a persistent kernel, whole in one CTA each or -- from
  * opts->conv_split points -- as phase tasks spread over many CTAs.  flags: 0,
  * or MUFFT_GB_FLAG_AUTOTUNE to time the batch with every split / class size
@@ -347,8 +347,8 @@ void mufft_gb_free_fft_batch(mufft_gb_fft_batch *batch);
 typedef struct mufft_gb_stream_conv mufft_gb_stream_conv;
 /* opts: NULL for the defaults.  opts->stream_conv_ranges: partition ranges
  * the multiply-accumulate splits the P partitions into (each range a row of
- * CTAs whose partial sums are added in range order; 0 sizes it to the GPU;
- * clamped to P, or P - 1 for one-launch blocks, which also keep every CTA
+ * CTAs whose partial sums are added in range order; 0 sizes it to the filter
+ * and the GPU; clamped to P, or P - 1 for one-launch blocks, which also keep every CTA
  * resident at once).  opts->stream_conv_fused: convolvers whose windows one
  * 256-thread row tile transforms (64 .. 4096 complex points) run a block as
  * one launch -- the forward transform, the multiply-accumulate and the
