@@ -27,17 +27,21 @@ __host__ __device__ constexpr int stage_table_base(int r, int p)
 {
     return (stage_radix_index(r) * kStageTableK + stage_p_offset(p)) * 4;
 }
-// Radix-32 stages (p in {16, 32, 256, 512}) follow, eight float2 for each k:
-// W^(e*k) for the exponents e below (the last one unused), so that every power
-// is a product of at most three.
-constexpr int kStage32Begin = 4 * kStageTableK * 4;
-constexpr int kStage32Exps[8] = {1, 2, 4, 8, 3, 12, 16, 0};
-constexpr int kStage32Sizes[4] = {16, 32, 256, 512};
-__host__ __device__ constexpr int stage32_base(int p)
+// The stages of schedules with radix 32 (fft_device.cuh, Sched) follow, ten
+// float2 for each k: W^(e*k) for the exponents e below (radix 16: the first
+// six), so that every power is one of them or a product of two.
+constexpr int kWideBegin = 4 * kStageTableK * 4;
+constexpr int kWideExps[10] = {1, 2, 3, 4, 8, 12, 16, 20, 24, 28};
+struct WideStage {
+    int r, p;
+};
+constexpr WideStage kWideStages[5] = {{16, 16}, {32, 16}, {32, 32}, {32, 256}, {32, 512}};
+// float2 index of a stage's table; past the last stage: the end
+__host__ __device__ constexpr int wide_base(int r, int p)
 {
-    return kStage32Begin + 8 * (p == 16 ? 0 : p == 32 ? 16 : p == 256 ? 48 : 304);
+    return kWideBegin + 10 * (r == 16 ? 0 : p == 16 ? 16 : p == 32 ? 32 : p == 256 ? 64 : p == 512 ? 320 : 832);
 }
-constexpr int kStageTableFloat2 = kStage32Begin + 8 * (16 + 32 + 256 + 512);
+constexpr int kStageTableFloat2 = wide_base(32, 0);
 
 // Thread-to-work decomposition of a CTA: which index runs fastest across
 // consecutive threads.  ALONG: consecutive threads walk along one transform

@@ -310,12 +310,12 @@ bool device_prepare(int *dev_out)
                         h[stage_table_base(r, p) + 4 * k + e] = make_float2((float)std::cos(ph), (float)std::sin(ph));
                     }
             }
-        for (int p : kStage32Sizes)
-            for (int k = 0; k < p; k++)
-                for (int e = 0; e < 8; e++) {
-                    const long long n = 32ll * p;
-                    double ph = -2.0 * M_PI * (double)(((long long)kStage32Exps[e] * k) % n) / (double)n;
-                    h[stage32_base(p) + 8 * k + e] = make_float2((float)std::cos(ph), (float)std::sin(ph));
+        for (const WideStage &w : kWideStages)
+            for (int k = 0; k < w.p; k++)
+                for (int e = 0; e < 10; e++) {
+                    const long long n = (long long)w.r * w.p;
+                    double ph = -2.0 * M_PI * (double)(((long long)kWideExps[e] * k) % n) / (double)n;
+                    h[wide_base(w.r, w.p) + 10 * k + e] = make_float2((float)std::cos(ph), (float)std::sin(ph));
                 }
         if (!cuda_ok(cudaMalloc(&ds.tw, h.size() * sizeof(float2)), "cudaMalloc(twiddles)"))
             return false;

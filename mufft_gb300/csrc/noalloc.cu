@@ -51,7 +51,7 @@ __global__ void noalloc_fill_twiddles(float2 *t)
     const int n = kStageTableFloat2;
     for (int idx = blockIdx.x * blockDim.x + threadIdx.x; idx < n; idx += gridDim.x * blockDim.x) {
         int r, p, k, e;
-        if (idx < kStage32Begin) {
+        if (idx < kWideBegin) {
             const int per_radix = kStageTableK * 4;
             const int ri = idx / per_radix;
             const int kk = (idx % per_radix) / 4;
@@ -60,11 +60,11 @@ __global__ void noalloc_fill_twiddles(float2 *t)
             p = kk < 16 ? 16 : (kk < 272 ? 256 : 4096);
             k = kk - stage_p_offset(p);
         } else {
-            constexpr int exps[8] = {1, 2, 4, 8, 3, 12, 16, 0};  // kStage32Exps
-            e = exps[(idx - kStage32Begin) % 8];
-            r = 32;
-            p = idx < stage32_base(32) ? 16 : idx < stage32_base(256) ? 32 : idx < stage32_base(512) ? 256 : 512;
-            k = (idx - stage32_base(p)) / 8;
+            constexpr int exps[10] = {1, 2, 3, 4, 8, 12, 16, 20, 24, 28};  // kWideExps
+            e = exps[(idx - kWideBegin) % 10];
+            r = idx < wide_base(32, 16) ? 16 : 32;
+            p = idx < wide_base(32, 32) ? 16 : idx < wide_base(32, 256) ? 32 : idx < wide_base(32, 512) ? 256 : 512;
+            k = (idx - wide_base(r, p)) / 10;
         }
         const long long rp = (long long)r * p;
         const long long m = ((long long)e * k) % rp;
