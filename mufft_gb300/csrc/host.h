@@ -27,6 +27,7 @@
 #include "../../include/mufft_gb300.h"
 #include "bc_fused.h"
 #include "common.h"
+#include "host_range.h"
 #include "registry.h"
 #include "split_tc.h"
 #include "tiles_persist.h"

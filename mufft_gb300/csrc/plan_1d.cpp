@@ -304,12 +304,37 @@ static Residence residence(const void *p)
     return {false, at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr};
 }
 
+// Whether `bytes` bytes from p on lie in one page-locked allocation or
+// registration.  A caller may have page-locked only part of a buffer: the
+// kernels could not reach the rest, a staged copy can (or reports an error).
+static bool page_locked(const void *p, size_t bytes)
+{
+    typedef CUresult (*GetAttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
+    static const GetAttributesFn get = [] {
+        void *f = nullptr;
+        cudaDriverEntryPointQueryResult q;
+        if (cudaGetDriverEntryPointByVersion("cuPointerGetAttributes", &f, 12000, cudaEnableDefault, &q) !=
+                cudaSuccess ||
+            q != cudaDriverEntryPointSuccess) {
+            cudaGetLastError();
+            return (GetAttributesFn) nullptr;
+        }
+        return (GetAttributesFn)f;
+    }();
+    CUdeviceptr start = 0;
+    size_t size = 0;
+    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[2] = {&start, &size};
+    return get && get(2, what, to, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS &&
+           range_holds((uintptr_t)start, size, (uintptr_t)p, bytes);
+}
+
 // Whether a blocking execute lets the kernel read and write the caller's
-// page-locked memory itself instead of staging it: one pass, which reads and
-// writes every element once, small buffers -- a copy each way costs more than
-// the link's latency (stereo block convolution of 2048 frames, input and
-// output call: 48.0 -> 26.5 us, mono 4096 55.0 -> 28.1) -- of the kernels' alignment, and apart from
-// each other (staging also serves transforms in place).
+// page-locked memory itself instead of staging it: one pass, small buffers -- a
+// copy each way costs more than the link's latency (stereo block convolution of
+// 2048 frames, input and output call: 48.0 -> 26.5 us, mono 4096 55.0 -> 28.1) --
+// page-locked as a whole, of the kernels' alignment, and apart from each other
+// (staging also serves transforms in place).
 constexpr size_t kDirectHostBytes = (size_t)1 << 20;
 
 static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out, const void *in2,
@@ -326,6 +351,9 @@ static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out
             return false;
     const uintptr_t i = (uintptr_t)in, o = (uintptr_t)out, i2 = (uintptr_t)in2;
     if ((i | o | i2) & 7)
+        return false;
+    if ((!rin.device && !page_locked(in, ib)) || (!rout.device && !page_locked(out, ob)) ||
+        (!rin2.device && !page_locked(in2, ib)))
         return false;
     auto apart = [](uintptr_t a, size_t an, uintptr_t c, size_t cn) { return a + an <= c || c + cn <= a; };
     return apart(i, ib, o, ob) && (!in2 || apart(i2, ib, o, ob));
