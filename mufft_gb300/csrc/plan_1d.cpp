@@ -335,8 +335,6 @@ static bool page_locked(const void *p, size_t bytes)
 // 2048 frames, input and output call: 48.0 -> 26.5 us, mono 4096 55.0 -> 28.1) --
 // page-locked as a whole, of the kernels' alignment, and apart from each other
 // (staging also serves transforms in place).
-constexpr size_t kDirectHostBytes = (size_t)1 << 20;
-
 static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out, const void *in2,
                         const Residence &rin, const Residence &rout, const Residence &rin2)
 {
@@ -344,7 +342,8 @@ static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out
         pl->passes[0].tk)
         return false;
     const size_t ib = pl->in_total(), ob = pl->out_total();
-    if (ib > kDirectHostBytes || ob > kDirectHostBytes)
+    const size_t most = direct_host_bytes(pl->M, pl->kind != K_C2C);
+    if (ib > most || ob > most)
         return false;
     for (const Residence *r : {&rin, &rout, &rin2})
         if (!r->device && !r->mapped)

@@ -72,3 +72,33 @@ def test_partly_page_locked(part, which):
     gpu.free_plan_1d(plan)
     src.close()
     dst.close()
+
+
+@pytest.mark.parametrize("kind, n, limit", [(0, 16, 1 << 18), (0, 32, 1 << 19), (1, 16, 1 << 18), (2, 32, 1 << 18),
+                                            (2, 64, 1 << 19), (0, 64, 1 << 20)])
+def test_limits_of_direct_access(kind, n, limit):
+    """The last batch the kernel takes itself and the first one that is staged: the same bits."""
+    import torch
+
+    import mufft_gb300
+    gpu = mufft_gb300.load()
+    fin, fout = (2 * n, n, n + 2)[kind], (2 * n, n + 2, n)[kind]  # floats per transform
+    most = limit // (4 * max(fin, fout))
+    for batch in (most, most + 1):
+        x = signals.uniform(85000 + n, fin * batch).astype(np.float32)
+        dx = torch.from_numpy(x).cuda()
+        dy = torch.empty(fout * batch, device="cuda")
+        plan = gpu.gb_create_plan_1d(kind, n, K.FORWARD, 0, batch, 0, 0, None)
+        assert plan
+        assert gpu.gb_execute_plan_1d_async(plan, dy.data_ptr(), dx.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+        want = dy.cpu().numpy()
+        src, dst = gpu.alloc(x.nbytes), gpu.alloc(want.nbytes)
+        assert gpu.gb_memcpy(src, dx.data_ptr(), x.nbytes) == 0
+        gpu.execute_plan_1d(plan, dst, src)
+        gpu.check("execute_plan_1d")
+        got = torch.empty(fout * batch, device="cuda")
+        assert gpu.gb_memcpy(got.data_ptr(), dst, want.nbytes) == 0
+        assert np.array_equal(got.cpu().numpy().view(np.uint32), want.view(np.uint32))
+        gpu.free_plan_1d(plan)
+        gpu.free(src)
+        gpu.free(dst)
