@@ -26,8 +26,7 @@ struct mufft_plan_conv {
     float2 *adj_spec = nullptr;              // spectra of the gradients
     size_t adj_spec_bytes = 0;
     float2 *adj_acc = nullptr;               // N/2 + 1 bins of the filter gradient
-    void *adj_part = nullptr;                // rows of partial sums of the reduction over signals
-    size_t adj_part_bytes = 0;
+    float2 *adj_part = nullptr;              // rows of partial sums of the reduction over signals
     // batched forms (mufft_gb_execute_conv_output_batched, mufft_gb_conv_adjoint):
     // plans over a chunk of signals and over the ragged last chunk
     struct BatchPlan {
@@ -173,6 +172,13 @@ bool conv_stereo(const mufft_plan_conv *c) { return (c->method & 1u) == MUFFT_CO
 // Spectrum bins of one gradient block: N/2 + 1 (mono r2c) or N (stereo).
 size_t conv_bins(const mufft_plan_conv *c) { return conv_stereo(c) ? c->N : c->N / 2 + 1; }
 
+int conv_sms(const mufft_plan_conv *c)
+{
+    int sms = 0;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
+    return sms;
+}
+
 bool conv_adj_spec(mufft_plan_conv *c, size_t bytes)
 {
     if (c->adj_spec_bytes >= bytes)
@@ -186,18 +192,28 @@ bool conv_adj_spec(mufft_plan_conv *c, size_t bytes)
     return true;
 }
 
+// The filter gradient's accumulator, and the partial sums of as many rows as
+// any number of signals takes: later calls with more signals leave both where
+// they are, in captured graphs too.
+bool conv_adj_acc(mufft_plan_conv *c)
+{
+    if (c->adj_acc)
+        return true;
+    const size_t row = (c->N / 2 + 1) * sizeof(float2);
+    const unsigned rows = adjoint_reduce_rows(c->N, ~0u, conv_sms(c));
+    if (rows > 1 && !c->adj_part && !cuda_ok(cudaMalloc(&c->adj_part, rows * row), "cudaMalloc(adjoint rows)"))
+        return false;
+    return cuda_ok(cudaMalloc(&c->adj_acc, row), "cudaMalloc");
+}
+
 // Sums the gradients' spectra of `n` signals (adj_spec) against their first
 // spectra into the filter gradient's bins.
 bool conv_reduce(mufft_plan_conv *c, const float2 *first, size_t dist, unsigned n, bool accumulate, cudaStream_t st)
 {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, c->device);
-    const unsigned rows = adjoint_reduce_rows(c->N, n, sms);
-    if (rows > 1 && !ensure(c->adj_part, c->adj_part_bytes, (size_t)rows * (c->N / 2 + 1) * sizeof(float2)))
-        return false;
-    return cuda_ok(launch_adjoint_filter_reduce(c->adj_acc, (float2 *)c->adj_part, rows, c->adj_spec,
-                                                (long long)conv_bins(c), first, (long long)dist, n, c->N,
-                                                conv_stereo(c) ? 1 : 0, 1.0f / (float)c->N, accumulate ? 1 : 0, st),
+    const unsigned rows = adjoint_reduce_rows(c->N, n, conv_sms(c));
+    return cuda_ok(launch_adjoint_filter_reduce(c->adj_acc, c->adj_part, rows, c->adj_spec, (long long)conv_bins(c),
+                                                first, (long long)dist, n, c->N, conv_stereo(c) ? 1 : 0,
+                                                1.0f / (float)c->N, accumulate ? 1 : 0, st),
                    "adjoint reduce");
 }
 
@@ -273,7 +289,7 @@ int mufft_gb_conv_adjoint_filter(mufft_plan_conv *plan, float *grad_filter, cons
         return t_err ? t_err : MUFFT_GB_ERR_ALLOC;
     if (!conv_adj_spec(plan, chunk * bins * sizeof(float2)))
         return t_err;
-    if (!plan->adj_acc && !cuda_ok(cudaMalloc(&plan->adj_acc, (N / 2 + 1) * sizeof(float2)), "cudaMalloc"))
+    if (!conv_adj_acc(plan))
         return t_err;
     const cudaStream_t st = (cudaStream_t)stream;
     const size_t elem = stereo ? sizeof(float2) : sizeof(float);  // one sample of a gradient block
@@ -420,7 +436,7 @@ int mufft_gb_conv_adjoint(mufft_plan_conv *plan, float *grad_filter, void *grad_
             plan->adj_c2r = create_1d(K_C2R, N, MUFFT_INVERSE, 0, 1, 0, 0, -1, false, nullptr);
         if (!plan->adj_c2r)
             return t_err ? t_err : MUFFT_GB_ERR_ALLOC;
-        if (!plan->adj_acc && !cuda_ok(cudaMalloc(&plan->adj_acc, (N / 2 + 1) * sizeof(float2)), "cudaMalloc"))
+        if (!conv_adj_acc(plan))
             return t_err;
     }
     const float2 *A = (const float2 *)first_spectra;
