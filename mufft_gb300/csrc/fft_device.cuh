@@ -930,11 +930,11 @@ __device__ __forceinline__ void run_stages(float2 (&v)[R], int j, int &c, int &t
 
 // Threads of one CTA, and the CTAs per SM the register budget is sized for:
 // 16-element tiles are held to 64 registers so that 1024 threads fit, 32-element
-// ones to 128 (512 threads).
+// ones to 128 (512 threads; LEAN: 96, 640 threads).
 template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_threads() { return C * (L / (R * Q)); }
-template <int L, int R, int C, int Q> __host__ __device__ constexpr int tile_min_blocks()
+template <int L, int R, int C, int Q, bool LEAN = false> __host__ __device__ constexpr int tile_min_blocks()
 {
-    constexpr int most = R <= 16 ? 1024 : 512;  // 64, or 128 registers a thread
+    constexpr int most = R <= 16 ? 1024 : (LEAN ? 640 : 512);  // 64, or 96 or 128 registers a thread
     return tile_threads<L, R, C, Q>() >= most ? 1 : most / tile_threads<L, R, C, Q>();
 }
 
@@ -1254,8 +1254,9 @@ __device__ __forceinline__ void tile_body(const TileArgs &a, unsigned tile, int 
         cg::this_cluster().barrier_wait();
 }
 
-template <int L, int R, int C, int Q, int LMAP, int SMAP, int FL = FL_ANY>
-__global__ void __launch_bounds__(tile_threads<L, R, C, Q>(), tile_min_blocks<L, R, C, Q>()) tile_fft(const TileArgs a)
+template <int L, int R, int C, int Q, int LMAP, int SMAP, int FL = FL_ANY, bool LEAN = false>
+__global__ void __launch_bounds__(tile_threads<L, R, C, Q>(), tile_min_blocks<L, R, C, Q, LEAN>())
+    tile_fft(const TileArgs a)
 {
     extern __shared__ float2 smem[];
     dependent_start();
@@ -1325,6 +1326,8 @@ template <int L, int R, int C, int Q, int LMAP, int SMAP> constexpr TileFlavours
             }
         }
         if constexpr (LMAP == ALONG && SMAP == ALONG) {
+            if constexpr (L == 512 && R == 32)
+                f.plain_many = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_PLAIN, true>;
             f.half_plain = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_HALF_PLAIN>;
             f.half_r2c = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_HALF_R2C>;
             f.mul_plain = (const void *)&tile_fft<L, R, C, Q, LMAP, SMAP, FL_MUL_PLAIN>;

@@ -11,6 +11,7 @@ namespace mgb {
 // Flavour), named by them.
 struct TileFlavours {
     const void *plain = nullptr;   // plain stores
+    const void *plain_many = nullptr;  // the same in fewer registers, for launches of many CTAs
     const void *colpow = nullptr;  // four-step twiddle by column powers
     const void *byrow = nullptr;   // four-step twiddle by grid row
     const void *r2c = nullptr;     // r2c fix-up, M + 1 bins

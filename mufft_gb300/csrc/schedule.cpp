@@ -204,7 +204,15 @@ static const void *tile_fn(const Pass &p)
     const bool byrow = a.epilogue == EPI_TWIDDLE && a.tw_by_y;
     const bool colpow = a.epilogue == EPI_TWIDDLE && !a.tw_by_y && a.tw_colpow;
     const void *f = nullptr;
-    if (a.prologue == PRO_PLAIN && !a.half)
+    // Rows of 512 points use 104 registers a thread: 19 CTAs fit an SM.  With more
+    // CTAs than that the form of 96 is faster, at the speed of HBM (c2c 512 x 32768
+    // 40.9 -> 39.8 us, x 8192 9.0 -> 8.6); below, its later twiddle loads cost more
+    // (x 1000 2.70 against 3.06).
+    constexpr unsigned long long kMany = 19 * 152;
+    if (fl.plain_many && plain && a.prologue == PRO_PLAIN && !a.half &&
+        (unsigned long long)p.grid.x * p.grid.y > kMany)
+        f = fl.plain_many;
+    else if (a.prologue == PRO_PLAIN && !a.half)
         f = plain ? fl.plain : (r2c ? fl.r2c : (byrow ? fl.byrow : (colpow ? fl.colpow : nullptr)));
     else if (a.prologue == PRO_PLAIN)
         f = plain ? fl.half_plain : (r2c ? fl.half_r2c : (colpow ? fl.half_colpow : nullptr));

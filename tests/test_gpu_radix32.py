@@ -61,3 +61,20 @@ def test_error_no_larger_than_radix_16(gpu, torch, N, batch, wide, narrow):
     x = torch.from_numpy(signals.complex_uniform(83000 + batch, batch * N).reshape(batch, N)).cuda()
     exact = torch.fft.fft(x.to(torch.complex128))
     assert _error(gpu, torch, N, batch, wide, x, exact) <= _error(gpu, torch, N, batch, narrow, x, exact)
+
+
+@pytest.mark.parametrize("ctas", [2887, 2888, 2889])
+@pytest.mark.parametrize("direction", [K.FORWARD, K.INVERSE])
+def test_rows_of_512_in_many_ctas(gpu, torch, ctas, direction):
+    """Both sides of the line between the two register budgets, ragged last tile."""
+    N, batch = 512, 2 * ctas - 1
+    x = torch.from_numpy(signals.complex_uniform(84000 + ctas, batch * N).reshape(batch, N)).cuda()
+    w = x.to(torch.complex128)
+    exact = torch.fft.fft(w) if direction == K.FORWARD else torch.fft.ifft(w) * N
+    p = gpu.gb_create_plan_1d(0, N, direction, 0, batch, 0, 0, None)
+    y = torch.empty_like(x)
+    assert gpu.gb_execute_plan_1d_async(p, y.data_ptr(), x.data_ptr(), torch.cuda.current_stream().cuda_stream) == 0
+    torch.cuda.synchronize()
+    gpu.free_plan_1d(p)
+    err = (y.to(torch.complex128) - exact).norm(dim=1) / exact.norm(dim=1)
+    assert float(err.max()) <= 2.0 ** -23 * 9  # eps * log2(N), every row
