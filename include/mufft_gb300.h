@@ -105,7 +105,8 @@ typedef struct mufft_gb_options {
     int split_engine;
     /* 2D columns: 0 automatic (8192 points and more as a two-pass four-step
      * of short, wide column tiles, and 4096 points for grids at least 4096
-     * (real) or 8192 (c2c) wide), 1 one pass, 2 two passes where possible */
+     * (real) or 8192 (c2c) wide with l2_residency on, or with fewer than 400
+     * columns to transform), 1 one pass, 2 two passes where possible */
     int columns_2d;
     /* ragged convolution batches: requests of at least conv_split complex
      * points run as phase tasks over many CTAs (0: none), of at least
@@ -127,7 +128,7 @@ typedef struct mufft_gb_options {
      * tiles wherever the tile has that variant (the 1024-thread 4096-point
      * column tile): -1 automatic (on), 0 off, 1 on */
     int persistent_tiles;
-    /* three-level transforms: the intermediate kept in L2 where it fits
+    /* multi-pass transforms: the intermediate kept in L2 where it fits
      * (stores marked evict-last, the input and output streamed evict-first,
      * the intermediate dropped from L2 without write-back once the last pass
      * has read it): -1 automatic, 0 off, 1 on */

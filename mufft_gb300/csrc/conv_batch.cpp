@@ -70,8 +70,6 @@ void destroy_conv_batch(mufft_gb_conv_batch *b)
     delete b;
 }
 
-// Task list for a split size, uploaded with the request table, and the graph
-// (counter resets + the persistent launch) that replays it.
 // Launches of one class pipeline on `st`.
 bool enqueue_class(mufft_gb_conv_batch *b, unsigned lg, bool stereo, bool zp, const ClassEntry *tab, unsigned K,
                    cudaStream_t st)
@@ -104,6 +102,9 @@ bool enqueue_class(mufft_gb_conv_batch *b, unsigned lg, bool stereo, bool zp, co
            cuda_ok(cudaLaunchKernel(i2.fn, dim3(L2 / i2.C, K), dim3(i2.threads), a2, i2.smem, st), "class launch");
 }
 
+// Task list for a split size, uploaded with the request table, and the graph
+// (counter resets, the classes' branches and the persistent launch) that
+// replays it.
 bool conv_batch_build(mufft_gb_conv_batch *b, unsigned split_lg, unsigned class_lg, unsigned small_grid)
 {
     DeviceGuard g(b->device);

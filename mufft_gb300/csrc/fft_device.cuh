@@ -1,5 +1,5 @@
 // Device building blocks of the GB300 FFT: complex arithmetic, register DFTs
-// of size 2/4/8/16 and the tile-FFT kernel template used by every pass.
+// of size 2/4/8/16/32 and the tile-FFT kernel template used by every pass.
 //
 // Algorithm (the GPU form of muFFT's Stockham autosort passes,
 // kernel.c:151-453): a transform of length L is a sequence of radix-r
@@ -208,7 +208,7 @@ constexpr int ilog2c(int n) { return n <= 1 ? 0 : 1 + ilog2c(n >> 1); }
 // Stage plan of a length-L transform whose threads own R elements each:
 // radix-16 stages, then one smaller stage for the leftover factor; threads of
 // 32 elements take radix-32 stages last where that saves a stage (and its
-// exchange through shared memory): 512 = 16 x 32,
+// exchange through shared memory): 512 = 16 x 32, 1024 = 32 x 32,
 // 8192 = 16 x 16 x 32, 16384 = 16 x 32 x 32.
 template <int L, int R> struct Sched {
     static_assert(L >= 2 && (L & (L - 1)) == 0, "power of two");
@@ -477,9 +477,6 @@ template <int V> struct Int {
     static constexpr int value = V;
 };
 
-// Stage-0 load: register u*r + m <- element p = j*B + tl + TL*u + m*Q*B of
-// transform `tr`.  ALONG loads have unit stride (the planner only builds them
-// that way), so addresses are a base plus constant offsets.
 // Start of a kernel launched by launch_dependent (launch.h): waits until the
 // stream's previous kernel has finished and its writes are visible.  Every CTA
 // of such a kernel passes here before it touches memory that another kernel
@@ -547,8 +544,7 @@ __device__ __forceinline__ void st_policy(float2 *p, float2 v, unsigned long lon
 
 // Flavours of a tile kernel: which prologue and epilogue it carries.  FL_ANY
 // decides both at run time, with every form compiled in; the others fix them,
-// so that a launch pays no per-element tests and holds less code.  All of
-// them read whole plain inputs (PRO_PLAIN, no `half`).
+// so that a launch pays no per-element tests and holds less code.
 // A form is a prologue, whether the input is zero-padded, an epilogue and the
 // four-step twiddle it applies (1: column powers, 2: by grid row).
 __host__ __device__ constexpr int form(int prologue, int half, int epilogue, int twiddle = 0)
@@ -591,6 +587,9 @@ template <int FL> __device__ __forceinline__ bool fl_colpow(const TileArgs &a)
     return FL == FL_ANY ? a.tw_colpow != 0 : FL >> 6 == 1;
 }
 
+// Stage-0 load: register u*r + m <- element p = j*B + tl + TL*u + m*Q*B of
+// transform `tr`.  ALONG loads have unit stride (the planner only builds them
+// that way), so addresses are a base plus constant offsets.
 template <int L, int R, int Q, int LMAP, bool COH = false, int FL = FL_ANY>
 __device__ __forceinline__ void load_stage0(const TileArgs &a, const float2 *__restrict__ in,
                                             const float2 *__restrict__ in2, unsigned tr, int j, int tl,

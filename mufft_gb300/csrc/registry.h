@@ -52,7 +52,7 @@ const TileKernel *find_tile(int L, int lmap, int smap, int C = 0, int R = 0, int
 // The instantiation for a pass of `rows` grid rows of `ntrans` transforms:
 // find_tile's where the plan's options prefer one (or ask for a form that
 // only some tiles have), else the measured choice for the pass's size.
-// real: a row pass with an r2c or c2r fix-up.
+// real: the one pass of a batch of r2c or c2r transforms (with the fix-up).
 const TileKernel *choose_tile(int L, int lmap, int smap, unsigned long long ntrans, unsigned long long rows,
                               bool real = false);
 

@@ -28,7 +28,8 @@ namespace mgb {
 namespace {
 
 constexpr unsigned kAny = ~0u;
-// two CTAs per SM: below, a narrower tile spreads the pass over more SMs
+// two CTAs per SM of GB300's 152 (described schedules, made without a device,
+// are those of the plans): below, a narrower tile spreads the pass over more SMs
 constexpr unsigned kFill = 2 * 152;
 
 struct TileRule {
@@ -39,7 +40,7 @@ struct TileRule {
 const TileRule kTileRules[] = {
     // Rows: one or two warps per tile.  Their barriers hold back fewer threads,
     // and the SMs are filled more evenly: 2^24 points as rows of 512 c2c / r2c /
-    // c2r 44.9 / 53.2 / 56.5 -> 40.1 / 44.1 / 47.9 (also one exchange fewer, 16 x
+    // c2r 44.6 / 52.7 / 56.1 -> 39.8 / 42.6 / 46.6 (also one exchange fewer, 16 x
     // 32), of 256 41.2 / 44.9 / 46.9 -> 40.5 / 41.3 / 43.3, of 128 40.8 / 48.5 /
     // 50.7 -> 40.0 / 46.4 / 48.4, of 64 46.5 / 59.6 / 59.9 -> 45.3 / 57.4 / 58.1;
     // 2^18 points as rows of 16 .. 512 2.7-5.7 -> 2.6-3.3
@@ -50,9 +51,9 @@ const TileRule kTileRules[] = {
     {32, ALONG, ALONG, 64, 16, 0, kAny},
     {16, ALONG, ALONG, 64, 16, 0, kAny},
     // Columns: 32 elements a thread save an exchange at 512 (16 x 32) and 1024
-    // points (32 x 32).  c2c 2^20 x 32 203 -> 192, with the rows below 181;
-    // 2^18 x 64 94.0 -> 81.1 and 2^19 x 64 189 -> 162 with 16 columns, which
-    // need enough of them (2^19 x 3: 14.2 against 13.4 with 8)
+    // points (32 x 32).  c2c 2^20 x 32 203 -> 180 with the rows below; 2^18 x 64
+    // 93.9 -> 80.7 and 2^19 x 64 189 -> 161 with 16 columns, which need enough of
+    // them (2^19 x 3: 14.2 against 13.4 with 8)
     {512, ACROSS, ACROSS, 16, 32, 2 * kFill, kAny},
     {512, ACROSS, ACROSS, 8, 32, 0, 2 * kFill},
     {1024, ACROSS, ACROSS, 8, 32, 0, kAny},
@@ -63,7 +64,7 @@ const TileRule kTileRules[] = {
     // of four, 11.2 -> 13.4)
     {64, ACROSS, ACROSS, 32, 16, 0, kAny},
     {2048, ACROSS, ACROSS, 8, 16, 256, kAny},
-    // Rows stored transposed: 2^17 x 61 40.0 -> 36.3, 2^21 x 16 200.1 -> 196.0
+    // Rows stored transposed: 2^17 x 61 39.8 -> 35.4, 2^21 x 16 200.1 -> 196.2
     {256, ALONG, ACROSS, 8, 16, 0, kFill},
     {512, ALONG, ACROSS, 8, 32, 0, kAny},
     {1024, ALONG, ACROSS, 8, 32, 0, kAny},
@@ -87,8 +88,8 @@ const TileKernel *choose_tile(int L, int lmap, int smap, unsigned long long ntra
             if (const TileKernel *t = find_tile(L, lmap, smap, r.C, r.R, 1))
                 return t;
     // real rows of 1024 as 32 x 32 where there are enough of them (2048-real
-    // frames x 4096 r2c / c2r 15.4 / 16.9 -> 14.3 / 16.0, x 16384 47.1 -> 43.1,
-    // but x 300 2.6 -> 2.8)
+    // frames x 4096 r2c / c2r 12.4 / 13.3 -> 10.6 / 11.8, x 16384 46.6 / 49.9 ->
+    // 41.6 / 45.3, but x 300 2.6 -> 2.8)
     if (real && L == 1024 && lmap == ALONG && smap == ALONG && ctas >= 1024)
         if (const TileKernel *t = find_tile(L, lmap, smap, 1, 32, 1))
             return t;

@@ -11,9 +11,8 @@
 // half in shared memory, reads its mirror's and resolves both bins.
 //
 // It replaces a row pass with plain stores and an in-place fix-up sweep (16
-// bytes read and written per bin): r2c 61 x 2^18 55.7 -> 45.3
-// us, 64 x 2^16 28.6 -> 14.7 (with the tile choices), 100 x 2^19 247 -> 142.  Rows of up to
-// 512 points: from 1024 a 16-row tile fills an SM alone, and narrower ones
+// bytes read and written per bin): r2c 61 x 2^18 55.7 -> 45.8 us, 64 x 2^16 28.6 ->
+// 13.2 (with the tile choices), 100 x 2^19 247 -> 144.  Rows of up to 512 points: from 1024 a 16-row tile fills an SM alone, and narrower ones
 // store 32-byte segments.
 #include "fft_device.cuh"
 #include "tiles_r2c_rows.h"

@@ -1,6 +1,7 @@
-"""Tile kernels compiled for one prologue and epilogue against the kernels
-that decide both at run time: a zero-padded transform (the run-time form)
-equals the plain transform of the same input with its zeros written out.
+"""Tile kernels compiled for one prologue and epilogue: a zero-padded transform
+equals the plain transform of the same input with its zeros written out, each
+side a form of its own.  (The kernels that decide prologue and epilogue at run
+time: test_column_twiddle_forms, and test_gpu_runtime_forms.py.)
 
 Both sides round independently, each with a relative L2 error of at most
 about eps/2 * log2(N) (eps = 2^-23), so they may differ by eps * log2(N)."""
