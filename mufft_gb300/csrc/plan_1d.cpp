@@ -286,29 +286,23 @@ mufft_plan_1d *create_1d(int kind, unsigned N, int direction, unsigned flags, un
 }
 
 // Where a buffer lives: memory the device owns (or migrates), or page-locked
-// host memory and its device address (null: neither).
+// host memory, its device address (null: neither) and the allocation or
+// registration it lies in.
 struct Residence {
     bool device;
     void *mapped;
+    uintptr_t start;
+    size_t size;
+
+    // Whether `bytes` bytes from p on are page-locked.  A caller may have
+    // page-locked only part of a buffer: the kernels could not reach the rest,
+    // a staged copy can (or reports an error).
+    bool holds(const void *p, size_t bytes) const { return mapped && range_holds(start, size, (uintptr_t)p, bytes); }
 };
 
 static Residence residence(const void *p)
 {
-    cudaPointerAttributes at;
-    if (cudaPointerGetAttributes(&at, p) != cudaSuccess) {
-        cudaGetLastError();
-        return {false, nullptr};
-    }
-    if (at.type == cudaMemoryTypeDevice || at.type == cudaMemoryTypeManaged)
-        return {true, nullptr};
-    return {false, at.type == cudaMemoryTypeHost ? at.devicePointer : nullptr};
-}
-
-// Whether `bytes` bytes from p on lie in one page-locked allocation or
-// registration.  A caller may have page-locked only part of a buffer: the
-// kernels could not reach the rest, a staged copy can (or reports an error).
-static bool page_locked(const void *p, size_t bytes)
-{
+    // one driver call for all attributes; zeros for memory CUDA does not know
     typedef CUresult (*GetAttributesFn)(unsigned, CUpointer_attribute *, void **, CUdeviceptr);
     static const GetAttributesFn get = [] {
         void *f = nullptr;
@@ -321,12 +315,21 @@ static bool page_locked(const void *p, size_t bytes)
         }
         return (GetAttributesFn)f;
     }();
-    CUdeviceptr start = 0;
+    if (!get)
+        return {is_device_accessible(p), nullptr, 0, 0};
+    CUmemorytype type = (CUmemorytype)0;
+    unsigned managed = 0;
+    CUdeviceptr mapped = 0, start = 0;
     size_t size = 0;
-    CUpointer_attribute what[2] = {CU_POINTER_ATTRIBUTE_RANGE_START_ADDR, CU_POINTER_ATTRIBUTE_RANGE_SIZE};
-    void *to[2] = {&start, &size};
-    return get && get(2, what, to, (CUdeviceptr)(uintptr_t)p) == CUDA_SUCCESS &&
-           range_holds((uintptr_t)start, size, (uintptr_t)p, bytes);
+    CUpointer_attribute what[5] = {CU_POINTER_ATTRIBUTE_MEMORY_TYPE, CU_POINTER_ATTRIBUTE_IS_MANAGED,
+                                   CU_POINTER_ATTRIBUTE_DEVICE_POINTER, CU_POINTER_ATTRIBUTE_RANGE_START_ADDR,
+                                   CU_POINTER_ATTRIBUTE_RANGE_SIZE};
+    void *to[5] = {&type, &managed, &mapped, &start, &size};
+    if (get(5, what, to, (CUdeviceptr)(uintptr_t)p) != CUDA_SUCCESS)
+        return {false, nullptr, 0, 0};
+    if (type == CU_MEMORYTYPE_DEVICE || managed)
+        return {true, nullptr, 0, 0};
+    return {false, type == CU_MEMORYTYPE_HOST ? (void *)(uintptr_t)mapped : nullptr, (uintptr_t)start, size};
 }
 
 // Whether a blocking execute lets the kernel read and write the caller's
@@ -345,14 +348,11 @@ static bool direct_host(const mufft_plan_1d *pl, const void *in, const void *out
     const size_t most = direct_host_bytes(pl->M, pl->kind != K_C2C);
     if (ib > most || ob > most)
         return false;
-    for (const Residence *r : {&rin, &rout, &rin2})
-        if (!r->device && !r->mapped)
-            return false;
     const uintptr_t i = (uintptr_t)in, o = (uintptr_t)out, i2 = (uintptr_t)in2;
     if ((i | o | i2) & 7)
         return false;
-    if ((!rin.device && !page_locked(in, ib)) || (!rout.device && !page_locked(out, ob)) ||
-        (!rin2.device && !page_locked(in2, ib)))
+    if ((!rin.device && !rin.holds(in, ib)) || (!rout.device && !rout.holds(out, ob)) ||
+        (!rin2.device && !rin2.holds(in2, ib)))
         return false;
     auto apart = [](uintptr_t a, size_t an, uintptr_t c, size_t cn) { return a + an <= c || c + cn <= a; };
     return apart(i, ib, o, ob) && (!in2 || apart(i2, ib, o, ob));
@@ -366,7 +366,7 @@ int exec_1d(mufft_plan_1d *pl, void *out, const void *in, const void *in2, cudaS
     }
     DeviceGuard g(pl->device);
     const Residence rin = residence(in), rout = residence(out),
-                    rin2 = pl->uses_in2 ? residence(in2) : Residence{true, nullptr};
+                    rin2 = pl->uses_in2 ? residence(in2) : Residence{true, nullptr, 0, 0};
     bool hin = !rin.device, hin2 = !rin2.device, hout = !rout.device;
     if (!sync && (hin || hin2 || hout)) {
         set_error(MUFFT_GB_ERR_HOST_POINTER, "asynchronous execute needs device-accessible buffers");
